@@ -250,7 +250,8 @@ int gbntt_set_wait_limit(uint32_t polls);
 /* Setting the environment variable GBNTT_TUNE_LOG=1 prints the autotuner's
  * timing of every candidate configuration to stderr at batch creation;
  * GBNTT_TUNE_FORCE="<log2 coefficients per thread>,<CTAs per SM, 0 = default>"
- * pins the choice among the candidates (the timing launches still run). */
+ * pins the choice among the candidates (the timing launches still run), "tc"
+ * the tensor-core kernel (canonical int16 batches of n = 2^5 .. 2^10). */
 int gbntt_batch_query(const gbntt_batch* batch, int what, int64_t* value);
 int gbntt_batch_destroy(gbntt_batch* batch);
 

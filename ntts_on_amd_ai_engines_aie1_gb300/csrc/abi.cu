@@ -14,9 +14,11 @@
 #include "device.cuh"
 #include "plan_internal.h"
 #include "tables.h"
+#include "tc16.cuh"
 
 namespace gbntt {
 const void* bitrev_kernel_ptr();
+const void* tc16_kernel(int L, bool bitrev_in, bool bitrev_out);   // kernels_tc16.cu
 }
 
 using namespace gbntt;
@@ -35,6 +37,8 @@ struct gbntt_plan {
     KArgs base;            // constants shared by every launch
     int2* d_tab = nullptr;
     size_t tab_bytes = 0;
+    size_t tc_bytes = 0;   // tensor-core table behind it in the same allocation
+    const void* tc_fn = nullptr;   // tensor-core kernel (canonical int16, n = 2^5 .. 2^10)
     int device = 0;
     std::mutex stage_mu;   // serialises gbntt_execute_host on this plan
     void* d_stage = nullptr;
@@ -166,6 +170,20 @@ int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, c
             return n > 0 ? n : 1;
         }();
         const bool small = batch <= (uint64_t)sms;
+        if (p->tc_fn) {
+            const unsigned long long tiles = ((batch << p->hp.L) + TC_TILE - 1) / TC_TILE;
+            // a warp per tile; one-warp CTAs, which spread over the SMs, up to
+            // the resident count
+            const unsigned long long cap = (unsigned long long)TC_OCC * (unsigned)sms;
+            const int threads = tiles <= cap ? 32 : TC_CTA;
+            const unsigned grid = (unsigned)std::min(cap, (tiles * 32 + threads - 1) / threads);
+            int L = p->hp.L;
+            void* targs[] = {&a, &L};
+            e = launch_kernel(p->tc_fn, grid, threads, threads / 32 * TC_WARP_RING, targs, s, true);
+            if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
+            g_launches.fetch_add(1, std::memory_order_relaxed);
+            return GBNTT_OK;
+        }
         const KernelInfo& k = small && p->kl.fn ? p->kl : p->ki;
         const unsigned long long blocks = (batch + k.polys - 1) / k.polys;
         if (blocks > 0x7FFFFFFFull) return fail(GBNTT_ERR_ARG, "batch too large for one launch");
@@ -335,6 +353,8 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
     const bool packed = (p->fam == F_R2F16 || p->fam == F_R2I16 || p->fam == F_R4F16);
     const bool inverse = (kind == K_R2_I16_INV || kind == K_R2_I32_INV || kind == K_R4_I16_INV);
     std::vector<int32_t> dev_tab;
+    std::vector<uint32_t> tc_tab;
+    uint32_t tc_ke = 0, tc_corr = 0;
     if (canon) {
         // canonical families: (w, w') pairs computed on the device; the
         // four-step holds the column and row transforms' tables and the twist
@@ -346,7 +366,12 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
             n_twist = canon_twist_entries(cl.L1, cl.L2, cl.row_el);
         }
         p->tab_bytes = (n_cols + n_rows + n_twist) * sizeof(int2);
-        e = cudaMalloc(&p->d_tab, p->tab_bytes);
+        if (hp.elem_bytes == 2 && tc_supported(hp.L, hp.q)) {
+            tc_build(hp.L, hp.q, hp.root, inverse, (flags & FLAG_NATURAL_ORDER) != 0, (flags & FLAG_SCALE_NINV) != 0,
+                     tc_tab, &tc_ke, &tc_corr);
+            p->tc_bytes = tc_tab.size() * sizeof(uint32_t);
+        }
+        e = cudaMalloc(&p->d_tab, p->tab_bytes + p->tc_bytes);
         if (e == cudaSuccess && cl.cols) e = cudaMalloc(&p->d_err, 256);
         if (e != cudaSuccess) {
             if (p->d_tab) cudaFree(p->d_tab);
@@ -370,6 +395,9 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
         } else {
             e = make_canon_table(p->d_tab, hp.L, q32, (uint32_t)hp.root, inverse, 0);
         }
+        if (e == cudaSuccess && p->tc_bytes)
+            e = cudaMemcpyAsync(reinterpret_cast<char*>(p->d_tab) + p->tab_bytes, tc_tab.data(), p->tc_bytes,
+                                cudaMemcpyHostToDevice, 0);
         if (e == cudaSuccess) e = cudaStreamSynchronize(0);
         if (e != cudaSuccess) {
             cudaFree(p->d_tab);
@@ -422,6 +450,13 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
         const uint64_t ninv = (uint64_t)modinv((int64_t)hp.n, hp.q);
         a.ninv = (unsigned)ninv;
         a.ninv_q = (unsigned)((ninv << 32) / (uint64_t)hp.q);
+        if (p->tc_bytes) {
+            const bool natural = (flags & FLAG_NATURAL_ORDER) != 0;
+            a.tctab = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(p->d_tab) + p->tab_bytes);
+            a.tc_ke = (int)tc_ke;
+            a.tc_corr = (int)tc_corr;
+            p->tc_fn = tc16_kernel(hp.L, inverse && !natural, !inverse && !natural);
+        }
     }
     a.natural_in = ((flags & FLAG_NATURAL_ORDER) && inverse) ? 1 : 0;
     a.natural_out = ((flags & FLAG_NATURAL_ORDER) && !inverse) ? 1 : 0;
@@ -469,7 +504,7 @@ int gbntt_plan_query(const gbntt_plan* p, int what, int64_t* value) {
     case GBNTT_Q_ELEM_BYTES: *value = p->hp.elem_bytes; break;
     case GBNTT_Q_STAGES: *value = p->hp.stages; break;
     case GBNTT_Q_KIND: *value = p->hp.kind; break;
-    case GBNTT_Q_TABLE_BYTES: *value = (int64_t)p->tab_bytes; break;
+    case GBNTT_Q_TABLE_BYTES: *value = (int64_t)(p->tab_bytes + p->tc_bytes); break;
     default: return fail(GBNTT_ERR_ARG, "unknown query");
     }
     return GBNTT_OK;

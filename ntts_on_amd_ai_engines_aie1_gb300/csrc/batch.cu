@@ -12,6 +12,7 @@
 #include "../../include/gb300_ntt.h"
 #include "batch_kernel.cuh"
 #include "plan_internal.h"
+#include "tc_tables.h"
 
 using namespace gbntt;
 
@@ -193,12 +194,16 @@ int autotune(gbntt_batch* b) {
             if (p.layouts[c].ms >= 0.f && p.layouts[c].ms < p.layouts[best].ms) best = c;
         // GBNTT_TUNE_FORCE="<log2 coefficients per thread>,<CTAs per SM>" pins the
         // choice (the timing launches still run), e.g. to profile the kernel a
-        // normal run picks while a profiler slows every launch down
+        // normal run picks while a profiler slows every launch down; "tc" pins
+        // the tensor-core kernel
         if (const char* f = std::getenv("GBNTT_TUNE_FORCE")) {
             int el = -1, occ = -1;
-            if (std::sscanf(f, "%d,%d", &el, &occ) == 2)
+            if (std::strcmp(f, "tc") == 0) {
                 for (size_t c = 0; c < p.layouts.size(); ++c)
-                    if (p.layouts[c].cfg.elmax == el && p.layouts[c].cfg.occ == occ) {
+                    if (p.layouts[c].cfg.tc) best = c;
+            } else if (std::sscanf(f, "%d,%d", &el, &occ) == 2)
+                for (size_t c = 0; c < p.layouts.size(); ++c)
+                    if (!p.layouts[c].cfg.tc && p.layouts[c].cfg.elmax == el && p.layouts[c].cfg.occ == occ) {
                         best = c;
                         break;
                     }
@@ -207,8 +212,9 @@ int autotune(gbntt_batch* b) {
         if (const char* log = std::getenv("GBNTT_TUNE_LOG"); log && *log == '1')
             for (size_t c = 0; c < p.layouts.size(); ++c)
                 std::fprintf(stderr, "gbntt autotune: %s part, %d coefficients/thread, %d threads/CTA, %d CTAs/SM, "
-                             "families 0x%x: %.2f us%s\n", p.i32 ? "int32" : "int16", 1 << p.layouts[c].cfg.elmax,
+                             "families 0x%x%s: %.2f us%s\n", p.i32 ? "int32" : "int16", 1 << p.layouts[c].cfg.elmax,
                              p.layouts[c].cfg.cta, p.layouts[c].cfg.occ, p.layouts[c].cfg.set,
+                             p.layouts[c].cfg.tc ? ", tensor cores" : "",
                              1e3 * p.layouts[c].ms, c == best ? "  <- chosen" : "");
     }
     if (flush) cudaFree(flush);
@@ -367,11 +373,15 @@ int gbntt_batch_create(gbntt_batch** out, const gbntt_segment* segs, uint32_t ns
     for (int i = 0; i < b->nparts; ++i) {
         auto& part = b->parts[i];
         int maxL = 0;
-        for (const auto& pe : part.pending) maxL = std::max(maxL, pe.L);
+        bool tc = true;                 // every segment has a tensor-core form
+        for (const auto& pe : part.pending) {
+            maxL = std::max(maxL, pe.L);
+            tc = tc && pe.a.tctab;
+        }
         const BatchConfig* cfgs = nullptr;
         const int ncfg = part.i32 ? batch_configs_i32(&cfgs) : batch_configs_i16(&cfgs);
         auto covers = [&](const BatchConfig& c) {
-            return (c.set & part.fam_mask) == part.fam_mask && config_fits(c, maxL);
+            return (c.set & part.fam_mask) == part.fam_mask && (c.tc ? tc : config_fits(c, maxL));
         };
         for (int c = 0; c < ncfg; ++c)
             if (covers(cfgs[c])) {
@@ -410,13 +420,14 @@ int gbntt_batch_create(gbntt_batch** out, const gbntt_segment* segs, uint32_t ns
             sd.n = 1 << L;
             sd.elem_bytes = eb;
             sd.variant = variant_id(fam, L);
-            const int G = 1 << (L - batch_el(L, elmax));
-            sd.polys_per_tile = lay.cfg.cta / G;
+            sd.polys_per_tile = lay.cfg.tc ? TC_TILE >> L : lay.cfg.cta >> (L - batch_el(L, elmax));
             sd.tiles = ((long long)u.count + sd.polys_per_tile - 1) / sd.polys_per_tile;
             sd.tile0 = lay.total_tiles;
             lay.total_tiles += sd.tiles;
-            lay.stage_bytes = std::max(lay.stage_bytes, batch_stage_bytes(lay.cfg.cta, L, eb, elmax));
-            lay.smem = std::max(lay.smem, batch_xbuf_bytes(lay.cfg.cta, L, elmax));
+            if (!lay.cfg.tc) {
+                lay.stage_bytes = std::max(lay.stage_bytes, batch_stage_bytes(lay.cfg.cta, L, eb, elmax));
+                lay.smem = std::max(lay.smem, batch_xbuf_bytes(lay.cfg.cta, L, elmax));
+            }
             lay.segs.push_back(sd);
         }
       }
@@ -432,7 +443,7 @@ int gbntt_batch_create(gbntt_batch** out, const gbntt_segment* segs, uint32_t ns
             gbntt_batch::Layout& lay = *lp;
             const bool zc = (lp == &b->parts[i].zlay);     // one staging buffer instead of two
             lay.stage_bytes = (lay.stage_bytes + 127) & ~127;
-            lay.smem = SMEM_HEADER + (zc ? 1 : 2) * lay.stage_bytes + lay.smem;
+            if (!lay.cfg.tc) lay.smem = SMEM_HEADER + (zc ? 1 : 2) * lay.stage_bytes + lay.smem;
             const void* fn = zc ? lay.cfg.zfn : lay.cfg.fn;
             cudaError_t e = raise_smem_limit(fn, lay.smem);
             int per_sm = 0;

@@ -4,6 +4,7 @@
 // batch_c16_small.cu (compiled in parallel); the zero-copy forms in
 // batch_k16_zc.cu.
 #include "batch_kernel.cuh"
+#include "tc16.cuh"
 
 namespace gbntt {
 
@@ -15,6 +16,7 @@ const void* batch_kernels_i16_w16g(int el, int set, int occ);
 const void* batch_kernels_c16(int el, int set, int occ);
 const void* batch_kernels_c16_small(int el, int set, int occ, int cta);
 const void* batch_zc_kernel_c16(int set, int el);
+const void* batch_kernel_tc16();
 
 namespace {
 constexpr int R2 = (1 << F_R2F16) | (1 << F_R2I16);
@@ -26,6 +28,7 @@ constexpr int C16 = (1 << F_C16F) | (1 << F_C16I);   // canonical forward + inve
 struct Key {
     int el, set, occ;
     int cta = BATCH_CTA;
+    bool tc = false;
 };
 // 256-thread CTAs with 64, 32 or 16 coefficients per thread; the narrower
 // ones carry less unrolled code per variant and fit more CTAs per SM (occ:
@@ -35,6 +38,8 @@ struct Key {
 constexpr Key kKeys[] = {
     {6, R4, 0}, {5, R4, 0}, {6, R2, 0}, {5, R2, 0}, {6, R8, 0}, {5, R8, 0}, {5, ALL16, 0},
     {4, R4, 0}, {4, R4, 5}, {4, R4, 6}, {4, R2, 0}, {4, R2, 5}, {4, R8, 0}, {4, R8, 5}, {4, ALL16, 0},
+    // canonical families on the tensor cores (n = 2^5 .. 2^10)
+    {5, C16, TC_OCC, TC_CTA, true},
     // canonical families: 16 coefficients per thread at 4, 5 and 6 CTAs/SM, 32 at 3
     // and 4 (8 per thread at 8 CTAs/SM spilled at its 32-register budget)
     {4, C16, 6}, {4, C16, 5}, {4, C16, 0}, {5, C16, 0}, {5, C16, 4},
@@ -54,17 +59,19 @@ int batch_configs_i16(const BatchConfig** out) {
         for (int i = 0; i < kN; ++i) {
             const Key k = kKeys[i];
             const void* fn = nullptr;
-            if (k.cta != BATCH_CTA) {
+            if (k.tc) {
+                fn = batch_kernel_tc16();
+            } else if (k.cta != BATCH_CTA) {
                 fn = batch_kernels_c16_small(k.el, k.set, k.occ, k.cta);
             } else {
                 for (auto get : {batch_kernels_i16_w64, batch_kernels_i16_w32, batch_kernels_i16_w32g,
                                  batch_kernels_i16_w16, batch_kernels_i16_w16g, batch_kernels_c16})
                     if (!fn) fn = get(k.el, k.set, k.occ);
             }
-            const void* zfn = k.cta != BATCH_CTA ? nullptr
+            const void* zfn = k.tc || k.cta != BATCH_CTA ? nullptr
                               : k.set == C16 ? (k.occ == 0 ? batch_zc_kernel_c16(k.set, k.el) : nullptr)
                                              : batch_zc_kernel_i16(k.set, k.el);
-            kI16[i] = BatchConfig{false, k.el, k.set, fn, zfn, k.cta, k.occ};
+            kI16[i] = BatchConfig{false, k.el, k.set, fn, zfn, k.cta, k.occ, k.tc};
         }
         return true;
     }();

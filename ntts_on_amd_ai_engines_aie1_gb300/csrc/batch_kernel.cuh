@@ -70,22 +70,7 @@ __global__ void __launch_bounds__(CTA, OCC ? OCC : batch_min_blocks(I32, CTA, EL
     const int tid = threadIdx.x, lane = tid & 31;
     const long long total = b.total_tiles;
 
-    // Segment of tile t: the last segment whose first tile is <= t (tile0 does
-    // not decrease; segment 0 starts at tile 0), searched in [lo, nsegs), lo a
-    // segment known to start at or before t.
-    // seg_find: a whole warp, 32 candidates per round, so a round costs one
-    // load latency however many segments the batch has (a CTA's first tile).
-    auto seg_find = [&](long long t, int lo) {
-        int hi = b.nsegs;
-        while (hi - lo > 1) {
-            const int step = (hi - lo + 31) >> 5;
-            const int j = lo + step * lane;
-            const unsigned m = __ballot_sync(0xffffffffu, j < hi && __ldg(&b.segs[j].tile0) <= t);
-            lo += step * (31 - __clz(m));                 // lane 0 (j = lo) always qualifies
-            hi = min(hi, lo + step);
-        }
-        return lo;
-    };
+    // Segment of tile t: warp_seg_find (a CTA's first tile), then
     // seg_of: one thread; a CTA's tiles increase, so the common case is t still
     // in segment lo (one load); past it, a binary search
     auto seg_of = [&](long long t, int lo) {
@@ -127,7 +112,7 @@ __global__ void __launch_bounds__(CTA, OCC ? OCC : batch_min_blocks(I32, CTA, EL
         sh_failed = 0;
     }
     if (t0 < total) {
-        const int s0 = seg_find(t0, 0);
+        const int s0 = warp_seg_find(b, t0, 0, lane);
         if (tid == 0) {
             issue(t0, 0, s0);
             sh_pending[0] = 1;
@@ -307,10 +292,12 @@ struct BatchConfig {
     const void* zfn;   // zero-copy form (k_batch_zc), or nullptr
     int cta;           // threads per CTA
     int occ;           // resident CTAs per SM the registers are budgeted for (0: the default)
+    bool tc = false;   // the tensor-core kernel (tc16.cuh): its own tile size, no shared memory
 };
 
-// the configuration carries a transform of 2^L coefficients
-inline bool config_fits(const BatchConfig& c, int L) { return batch_fits(L, c.cta, c.elmax); }
+// the window/exchange configuration carries a transform of 2^L coefficients
+// (never true of the tensor-core one: batch.cu asks tc_supported)
+inline bool config_fits(const BatchConfig& c, int L) { return !c.tc && batch_fits(L, c.cta, c.elmax); }
 
 // the persistent launch of a batch part: storage type and arithmetic
 // (the reference's lanes or the canonical families) -- 4 parts

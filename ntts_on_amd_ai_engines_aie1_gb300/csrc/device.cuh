@@ -66,7 +66,10 @@ struct KArgs {
     int wq1;              // radix-4: multiplier of the twiddle 1 (table entry 0)
     int q;
     int c;                // Barrett constant of the reduction (K = 16 or 32)
-    int fneg, wc;         // radix-4 omega_4 and its multiplier
+    union {
+        struct { int fneg, wc; };          // radix-4 omega_4 and its multiplier
+        struct { int tc_ke, tc_corr; };    // tensor-core form: the constants of its start values (tc_build)
+    };
     int canonical;        // reduce outputs to [0, q)
     int canon_c;          // its Barrett constant round(2^32 / q)
     int natural_in;       // input in natural order (inverse designs): bit reversal fused into the load
@@ -83,7 +86,10 @@ struct KArgs {
     unsigned cq;          // floor(2^32 / q)
     int in_off;           // int16: 2M, M = q ceil(2^15 / q); int32: q - (2^31 mod q)
     unsigned ninv, ninv_q;   // n^-1 mod q and its Shoup quotient (n^-1 scaling of inverse designs)
-    const int2* twist;    // four-step row twist factors (two-pass canonical int32 transforms)
+    union {
+        const int2* twist;    // four-step row twist factors (two-pass canonical int32 transforms)
+        const uint4* tctab;   // canonical int16: the tensor-core form's table (tc16.cuh), or nullptr
+    };
 };
 
 // The scalar constants of one design, held in registers while a polynomial is

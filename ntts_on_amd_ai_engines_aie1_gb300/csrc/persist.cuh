@@ -51,6 +51,22 @@ constexpr unsigned BATCH_WAIT_POLLS = 1u << 22;
 __host__ __device__ constexpr int batch_el(int L, int elmax) { return L < elmax ? L : elmax; }
 __host__ __device__ constexpr int variant_id(int fam, int L) { return (fam << 4) | L; }
 
+// The segment of tile t: the last one whose first tile is <= t (tile0 does not
+// decrease; segment 0 starts at tile 0), searched by a whole warp in
+// [lo, nsegs), lo a segment known to start at or before t: 32 candidates per
+// round, so a round costs one load latency however many segments there are.
+__device__ __forceinline__ int warp_seg_find(const BatchDev& b, long long t, int lo, int lane) {
+    int hi = b.nsegs;
+    while (hi - lo > 1) {
+        const int step = (hi - lo + 31) >> 5;
+        const int j = lo + step * lane;
+        const unsigned m = __ballot_sync(0xffffffffu, j < hi && __ldg(&b.segs[j].tile0) <= t);
+        lo += step * (31 - __clz(m));                 // lane 0 (j = lo) always qualifies
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
 // ---------------------------------------------------------------------------
 // PTX wrappers: mbarrier and bulk (TMA) copies
 // ---------------------------------------------------------------------------
