@@ -440,6 +440,7 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
     a.canon_c = hp.q >= 3 ? (int)((((uint64_t)1 << 32) + hp.q / 2) / hp.q) : 0;
     if (canon) {
         a.canonical = 1;
+        a.c = (int)(2 * hp.q);
         a.cq = (unsigned)((((uint64_t)1) << 32) / (uint64_t)hp.q);
         if (hp.elem_bytes == 2) {
             const int64_t m = hp.q * ((32768 + hp.q - 1) / hp.q);     // a multiple of q, >= 2^15

@@ -65,7 +65,7 @@ struct KArgs {
     const int* tab16;     // int16 designs: tw | w' << 16 packed in one word
     int wq1;              // radix-4: multiplier of the twiddle 1 (table entry 0)
     int q;
-    int c;                // Barrett constant of the reduction (K = 16 or 32)
+    int c;                // Barrett constant of the reduction (K = 16 or 32); canonical families: 2q
     union {
         struct { int fneg, wc; };          // radix-4 omega_4 and its multiplier
         struct { int tc_ke, tc_corr; };    // tensor-core form: the constants of its start values (tc_build)
@@ -225,16 +225,17 @@ __host__ __device__ __forceinline__ int canon(int x, int q, int c) {
 __device__ __forceinline__ unsigned shoup_mul(unsigned y, unsigned w, unsigned wq, unsigned q) {
     return y * w - __umulhi(y, wq) * q;
 }
-// [0, 2m) -> [0, m) for an unsigned lane (x - m wraps to a large value when x < m)
-__device__ __forceinline__ unsigned lazy_sub(unsigned x, unsigned m) { return min(x, x - m); }
+// [0, 2m) -> [0, m) for an unsigned lane (x - m wraps to a large value when x <
+// m); one add-and-minimum instruction, which min(x, x - m) is not compiled to
+__device__ __forceinline__ unsigned lazy_sub(unsigned x, unsigned m) { return __viaddmin_u32(x, 0u - m, x); }
 
 // int32 input coefficient (any signed value) -> a lane in [0, 2q): x + 2^31 is
 // reduced by one Barrett step with floor(2^32 / q) (error below 2q), then the
 // residue of -2^31 is added back and the sum folded below 2q
-__device__ __forceinline__ unsigned canon_in32(int x, unsigned q, unsigned cq, unsigned k31) {
+__device__ __forceinline__ unsigned canon_in32(int x, unsigned q, unsigned q2, unsigned cq, unsigned k31) {
     const unsigned u = (unsigned)x ^ 0x80000000u;
     const unsigned r = u - __umulhi(u, cq) * q;
-    return lazy_sub(r + k31, 2u * q);
+    return lazy_sub(r + k31, q2);
 }
 // a lane below 2^32 -> [0, q)
 __device__ __forceinline__ unsigned canon_out(unsigned v, unsigned q, unsigned cq) {
@@ -295,9 +296,9 @@ __device__ __forceinline__ void epilogue(int (&v)[E], const KArgs& a) {
 template <int FAM, int E>
 __device__ __forceinline__ void prologue(int (&v)[E], const KArgs& a) {
     if constexpr (FAM == F_C32F || FAM == F_C32I) {
-        const unsigned q = (unsigned)a.q, cq = a.cq, k31 = (unsigned)a.in_off;
+        const unsigned q = (unsigned)a.q, q2 = (unsigned)a.c, cq = a.cq, k31 = (unsigned)a.in_off;
 #pragma unroll
-        for (int k = 0; k < E; ++k) v[k] = (int)canon_in32(v[k], q, cq, k31);
+        for (int k = 0; k < E; ++k) v[k] = (int)canon_in32(v[k], q, q2, cq, k31);
     }
 }
 
@@ -625,7 +626,9 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
             // registers) or consecutive entries (j from the lane index).
             static_assert(!HIB, "the canonical families run whole sub-transforms (the four-step twist is separate)");
             const int k1 = k0 | (1 << KB);
-            const unsigned uq = (unsigned)q, q2 = uq << 1;
+            // 2q comes as a value of its own: from q, every x + 2q - y
+            // becomes a shift-and-add and a subtraction
+            const unsigned uq = (unsigned)q, q2 = (unsigned)a.c;
             if constexpr (topdown(FAM)) {
                 // Forward: Gentleman-Sande, natural order in, bit-reversed out.
                 // Layer S pairs the positions differing in bit B = L-1-S:
