@@ -349,8 +349,10 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
             return cuda_fail(e, "cudaFuncSetAttribute");
         }
     }
-    // int16 radix-2/4 designs: (tw, w') packed into one word (both fit int16)
-    const bool packed = (p->fam == F_R2F16 || p->fam == F_R2I16 || p->fam == F_R4F16);
+    // radix-4 and wide radix-2 int16 designs: (tw, w') packed into one word
+    // (both fit int16)
+    const int lean = p->fam == F_R2F16 || p->fam == F_R2I16 ? r2_form(hp.q, hp.c) : R2_WIDE;
+    const bool packed = lean == R2_WIDE && (p->fam == F_R2F16 || p->fam == F_R2I16 || p->fam == F_R4F16);
     const bool inverse = (kind == K_R2_I16_INV || kind == K_R2_I32_INV || kind == K_R4_I16_INV);
     std::vector<int32_t> dev_tab;
     std::vector<uint32_t> tc_tab;
@@ -436,6 +438,7 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
     a.c = hp.c;
     a.fneg = hp.r4_fneg;
     a.wc = hp.r4_wc;
+    if (p->fam == F_R2F16 || p->fam == F_R2I16) a.lean = lean;
     a.canonical = (flags & FLAG_CANONICAL) ? 1 : 0;
     a.canon_c = hp.q >= 3 ? (int)((((uint64_t)1 << 32) + hp.q / 2) / hp.q) : 0;
     if (canon) {

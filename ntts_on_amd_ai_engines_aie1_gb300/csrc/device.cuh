@@ -69,6 +69,7 @@ struct KArgs {
     union {
         struct { int fneg, wc; };          // radix-4 omega_4 and its multiplier
         struct { int tc_ke, tc_corr; };    // tensor-core form: the constants of its start values (tc_build)
+        int lean;                          // radix-2 int16: form of the butterflies (R2_WIDE ...)
     };
     int canonical;        // reduce outputs to [0, q)
     int canon_c;          // its Barrett constant round(2^32 / q)
@@ -127,12 +128,23 @@ __device__ __forceinline__ KC make_kc(const KArgs& a) {
 // lane arithmetic
 // ---------------------------------------------------------------------------
 
-// round(p / 2^16), ties toward zero (SRS, symmetric_zero)
-__device__ __forceinline__ int rsz16(int p) { return (p + 0x7FFF + (int)((unsigned)p >> 31)) >> 16; }
+// round(a b / 2^16), ties toward zero (SRS, symmetric_zero), for int16 a and b:
+// floor((p + 0x7FFF + [p < 0]) / 2^16) with p = a b.  The bias rides in the
+// product's addend and the sign is read after it, which makes the sum
+// x + (x >>> 31) one instruction: for -0x7FFF <= p < 0, where the bias hides the
+// sign, both forms give 0.
+__host__ __device__ __forceinline__ int rsz16(int a, int b) {
+    const int p = a * b + 0x7FFF;
+    return (p + (int)((unsigned)p >> 31)) >> 16;
+}
 
-// round(p / 2^32), ties toward zero
-__host__ __device__ __forceinline__ int rsz32(long long p) {
-    return (int)((p + 0x7FFFFFFFLL + (long long)((unsigned long long)p >> 63)) >> 32);
+// round(a b / 2^32), ties toward zero: the high word of a b + 0x7FFFFFFF +
+// [a b < 0].  The sign is a's xor b's (either where the product is 0: 2^31 has
+// the high word 0 too), known before the product, so bias and sign are its
+// 64-bit addend instead of a 64-bit addition behind it.
+__host__ __device__ __forceinline__ int rsz32(int a, int b) {
+    const unsigned bias = 0x7FFFFFFFu + ((unsigned)(a ^ b) >> 31);
+    return (int)(((long long)a * b + (long long)(unsigned long long)bias) >> 32);
 }
 
 // round(p / 2^31), ties toward zero
@@ -151,21 +163,42 @@ __device__ __forceinline__ int hi16(int w) { return w >> 16; }
 // within 1.5 of w 2^16 / q (0.5 for the float and constant ones, < 1.5 for
 // round<T>'s truncation of negative values), so for |a| <= 2^15 the quotient
 // error is at most 0.5 + 0.75 and |result| <= 1.25 q < 2^15 for q < 2^16 / 3.
-__device__ __forceinline__ int br16(int a, int c, int q) { return a - rsz16(a * c) * q; }
-__device__ __forceinline__ int bm16(int a, int tw, int wq, int q) { return a * tw - rsz16(a * wq) * q; }
+__host__ __device__ __forceinline__ int br16(int a, int c, int q) { return a - rsz16(a, c) * q; }
+__host__ __device__ __forceinline__ int bm16(int a, int tw, int wq, int q) { return a * tw - rsz16(a, wq) * q; }
+// br16 for an odd constant c: a c = 2^15 mod 2^16 only at a = -2^15, where
+// rounding up is toward zero, so plain rounding (half up) is the same
+__host__ __device__ __forceinline__ int br16_odd(int a, int c, int q) { return a - ((a * c + 0x8000) >> 16) * q; }
 // The same product when only its low 16 bits are used (it feeds sums that are
 // wrapped to int16): the packed table word t = (tw & 0xFFFF) | (w' << 16)
 // multiplies like tw modulo 2^16, so tw need not be sign-extended out of it.
 __device__ __forceinline__ unsigned bm16_lo(int a, int t, int q) {
-    return (unsigned)a * (unsigned)t - (unsigned)rsz16(a * hi16(t)) * (unsigned)q;
+    return (unsigned)a * (unsigned)t - (unsigned)rsz16(a, hi16(t)) * (unsigned)q;
+}
+
+// Forms of the radix-2 int16 butterflies, u +- w with u = br16, |u| <= 0.75 q
+// (c within 0.5 of 2^16 / q), and w = bm16, |w| <= 1.25 q:
+//   R2_WIDE     any modulus: the results are wrapped to int16 lanes;
+//   R2_LEAN     q < 2^14: |u +- w| <= 2 q < 2^15, the wrap changes nothing and
+//               is left out (w is exact then: the table holds tw and w' apart);
+//   R2_LEAN_ODD and an odd c (12289, 7681): br16_odd.
+enum { R2_WIDE = 0, R2_LEAN = 1, R2_LEAN_ODD = 2 };
+__host__ __device__ constexpr int r2_form(long long q, int c) {
+    return q >= 16384 ? R2_WIDE : c & 1 ? R2_LEAN_ODD : R2_LEAN;
+}
+template <int FORM>
+__device__ __forceinline__ void r2_butterfly16(int& x, int& y, int2 t, int c, int q) {
+    const int u = FORM == R2_LEAN_ODD ? br16_odd(x, c, q) : br16(x, c, q);
+    const int w = bm16(y, t.x, t.y, q);
+    x = u + w;
+    y = u - w;
 }
 
 // int32 variants, computed modulo 2^32 like the int32 lanes
 __host__ __device__ __forceinline__ int br32(int a, int c, int q) {
-    return (int)((unsigned)a - (unsigned)rsz32((long long)a * c) * (unsigned)q);
+    return (int)((unsigned)a - (unsigned)rsz32(a, c) * (unsigned)q);
 }
-__device__ __forceinline__ int bm32(int a, int tw, int wq, int q) {
-    return (int)((unsigned)a * (unsigned)tw - (unsigned)rsz32((long long)a * wq) * (unsigned)q);
+__host__ __device__ __forceinline__ int bm32(int a, int tw, int wq, int q) {
+    return (int)((unsigned)a * (unsigned)tw - (unsigned)rsz32(a, wq) * (unsigned)q);
 }
 __device__ __forceinline__ int add32(int a, int b) { return (int)((unsigned)a + (unsigned)b); }
 __device__ __forceinline__ int sub32(int a, int b) { return (int)((unsigned)a - (unsigned)b); }
@@ -180,7 +213,7 @@ __device__ __forceinline__ int r8red(int y, int tw, int wq, int q) {
 // Full Barrett multiplication by a constant, fully reduced
 // (src/kernels/full_reduction_kernels.cc:33-195).
 __device__ __forceinline__ int fb16(int x, int fs, int wq, int q) {
-    const int mb = wrap16(rsz16(x * wq));     // m' = SRS_16(x w'), symmetric_zero (:204-212)
+    const int mb = wrap16(rsz16(x, wq));     // m' = SRS_16(x w'), symmetric_zero (:204-212)
     const int r = x * fs - q * mb;            // x F_s - m' q (:234-238)
     const int lo = wrap16(r);                 // low 16 bits (:241)
     const int sign = wrap16(r >> 16);         // floor(r / 2^16) (:228, :242)
@@ -598,7 +631,7 @@ __device__ __forceinline__ void exchange_cols(int (&v)[1 << EL], int* sp, int g,
 // twiddle block index carries hi in its top bits.
 // fresh: no thread of the CTA has touched sp since the CTA's last barrier, so
 // the transform's first exchange needs no leading barrier (uniform)
-template <int FAM, int L, int EL, int S, int XC = 0, bool HIB = false>
+template <int FAM, int L, int EL, int S, int XC = 0, bool HIB = false, int FORM = R2_WIDE>
 __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const KC& a, int hi = 0, int cl = 0,
                                         bool fresh = false) {
     constexpr int E = 1 << EL;
@@ -691,7 +724,9 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
             // ntt_r2_kernels.cc:434-472, ntt_r2_int32_kernels.cc:267-295)
             const int k1 = k0 | (1 << KB);
             const int blk = ((HIB ? (hi << L) : 0) | posmap<LO, EL>(g, k0)) >> (B + 1);
-            if constexpr (FAM == F_R2F16) {
+            if constexpr (FAM == F_R2F16 && FORM != R2_WIDE) {
+                r2_butterfly16<FORM>(v[k0], v[k1], __ldg(&a.tab[blk]), a.c, q);
+            } else if constexpr (FAM == F_R2F16) {
                 const int t = __ldg(&a.tab16[blk]);
                 const unsigned u = (unsigned)br16(v[k0], a.c, q), w = bm16_lo(v[k1], t, q);
                 v[k0] = wrap16((int)(u + w));
@@ -717,6 +752,9 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
                 const int s = wrap16(v[k0] + v[k1]), d = wrap16(v[k0] - v[k1]);
                 v[k0] = s;
                 v[k1] = d;
+            } else if constexpr (FORM != R2_WIDE) {
+                r2_butterfly16<FORM>(v[k0], v[k1], __ldg(&a.tab[(1 << B) + (posmap<LO, EL>(g, k0) & ((1 << B) - 1))]), a.c,
+                                     q);
             } else {
                 const int tpos = posmap<LO, EL>(g, k0) & ((1 << B) - 1);
                 const int t = __ldg(&a.tab16[(1 << B) + tpos]);
@@ -816,9 +854,20 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
     }
 }
 
+// lean: the form of radix-2 int16 butterflies (the same for the whole CTA)
 template <int FAM, int L, int EL, int... S>
-__device__ __forceinline__ void run_steps(int (&v)[1 << EL], int* sp, int g, const KC& a, bool fresh,
+__device__ __forceinline__ void run_steps(int (&v)[1 << EL], int* sp, int g, const KC& a, int lean, bool fresh,
                                           std::integer_sequence<int, S...>) {
+    if constexpr (FAM == F_R2F16 || FAM == F_R2I16) {
+        if (lean == R2_LEAN_ODD) {
+            (do_step<FAM, L, EL, S, 0, false, R2_LEAN_ODD>(v, sp, g, a, 0, 0, fresh), ...);
+            return;
+        }
+        if (lean == R2_LEAN) {
+            (do_step<FAM, L, EL, S, 0, false, R2_LEAN>(v, sp, g, a, 0, 0, fresh), ...);
+            return;
+        }
+    }
     (do_step<FAM, L, EL, S>(v, sp, g, a, 0, 0, fresh), ...);
 }
 
@@ -992,7 +1041,7 @@ __device__ __forceinline__ void k_ntt_body(const KArgs& a) {
     }
     prologue<FAM>(v, a);
     const KC kc = make_kc(a);
-    run_steps<FAM, L, EL>(v, sp, g, kc, fresh, std::make_integer_sequence<int, NS>{});
+    run_steps<FAM, L, EL>(v, sp, g, kc, a.lean, fresh, std::make_integer_sequence<int, NS>{});
     epilogue<FAM, BR>(v, a);
     if constexpr (BR) {
         permute_br<L, EL, LOZ>(v, sp, g);

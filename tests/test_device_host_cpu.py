@@ -29,3 +29,7 @@ def test_exchange_layouts_conflict_free(tmp_path):
 
 def test_canonical_reduction(tmp_path):
     _run_host_check(tmp_path, "canon_reduce")
+
+
+def test_lane_rounding(tmp_path):
+    _run_host_check(tmp_path, "lane_rounding")
