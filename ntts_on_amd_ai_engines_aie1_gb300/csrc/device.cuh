@@ -626,6 +626,19 @@ __device__ __forceinline__ void exchange_cols(int (&v)[1 << EL], int* sp, int g,
     for (int k = 0; k < E; ++k) v[k] = sp[posmap<LOB, EL>(g, k) * XC + cl];
 }
 
+// the (w, w') pairs of one layer that a thread finds in consecutive entries of
+// the int2 table (0: none, or not worth a vector load): the block-indexed
+// designs' blocks of the thread's run, or the canonical families' entries
+// 2^B .. 2^(B+1) - 1, when the window is the lowest bits
+template <int FAM, int FORM>
+__host__ __device__ constexpr int step_vec_pairs(int LO, int EL, int B) {
+    if (LO != 0) return 0;
+    if (fam_canon(FAM)) return B >= 1 && B < EL ? 1 << B : 0;
+    const bool blocks = FAM == F_R2F32 || FAM == F_R2G32 || (FAM == F_R2F16 && FORM != R2_WIDE);
+    const int n = (1 << EL) >> (B + 1);
+    return blocks && n >= 2 ? n : 0;
+}
+
 // XC > 0: column pass (XC columns per CTA, exchanges through exchange_cols);
 // HIB: row pass, the polynomial is row `hi` of a longer transform and the
 // twiddle block index carries hi in its top bits.
@@ -649,6 +662,20 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
         }
     }
     const int q = a.q;
+    // In the window on the low bits the (w, w') pairs a thread needs in one
+    // layer are NV consecutive table entries: 16-byte loads take two at a time.
+    constexpr int NV = step_vec_pairs<FAM, FORM>(LO, EL, B);
+    int2 tv[NV > 0 ? NV : 1];
+    if constexpr (NV > 0) {
+        const int e0 = fam_canon(FAM) ? 1 << B : ((HIB ? (hi << L) : 0) | posmap<LO, EL>(g, 0)) >> (B + 1);
+        const int4* src = reinterpret_cast<const int4*>(a.tab + e0);
+#pragma unroll
+        for (int i = 0; i < NV / 2; ++i) {
+            const int4 w = __ldg(src + i);
+            tv[2 * i] = make_int2(w.x, w.y);
+            tv[2 * i + 1] = make_int2(w.z, w.w);
+        }
+    }
 #pragma unroll
     for (int r = 0; r < (E >> W); ++r) {
         const int k0 = ((r >> KB) << (KB + W)) | (r & ((1 << KB) - 1));
@@ -687,7 +714,8 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
                     d = x + ((unsigned)a.in_off << S) - y;
                 }
                 if constexpr (S != L - 1) {
-                    const int2 t = __ldg(&a.tab[(1 << B) + (posmap<LO, EL>(g, k0) & ((1 << B) - 1))]);
+                    const int2 t = NV > 0 ? tv[k0 & (NV - 1)]
+                                          : __ldg(&a.tab[(1 << B) + (posmap<LO, EL>(g, k0) & ((1 << B) - 1))]);
                     d = shoup_mul(d, (unsigned)t.x, (unsigned)t.y, uq);
                 }
                 v[k0] = (int)s;
@@ -712,7 +740,8 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
                 // the lane bound grows by 2q per layer (int16: below 2^20 after
                 // 12 layers); int32 lanes keep Harvey's bound, x < 2q before the
                 // butterfly and both outputs below 4q
-                const int2 t = __ldg(&a.tab[(1 << B) + (posmap<LO, EL>(g, k0) & ((1 << B) - 1))]);
+                const int2 t = NV > 0 ? tv[k0 & (NV - 1)]
+                                      : __ldg(&a.tab[(1 << B) + (posmap<LO, EL>(g, k0) & ((1 << B) - 1))]);
                 unsigned x = (unsigned)v[k0];
                 if constexpr (fam_i32(FAM)) x = lazy_sub(x, q2);
                 const unsigned m = shoup_mul((unsigned)v[k1], (unsigned)t.x, (unsigned)t.y, uq);
@@ -725,14 +754,14 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
             const int k1 = k0 | (1 << KB);
             const int blk = ((HIB ? (hi << L) : 0) | posmap<LO, EL>(g, k0)) >> (B + 1);
             if constexpr (FAM == F_R2F16 && FORM != R2_WIDE) {
-                r2_butterfly16<FORM>(v[k0], v[k1], __ldg(&a.tab[blk]), a.c, q);
+                r2_butterfly16<FORM>(v[k0], v[k1], NV > 0 ? tv[k0 >> (B + 1)] : __ldg(&a.tab[blk]), a.c, q);
             } else if constexpr (FAM == F_R2F16) {
                 const int t = __ldg(&a.tab16[blk]);
                 const unsigned u = (unsigned)br16(v[k0], a.c, q), w = bm16_lo(v[k1], t, q);
                 v[k0] = wrap16((int)(u + w));
                 v[k1] = wrap16((int)(u - w));
             } else {
-                const int2 t = __ldg(&a.tab[blk]);
+                const int2 t = NV > 0 ? tv[k0 >> (B + 1)] : __ldg(&a.tab[blk]);
                 const int u = br32(v[k0], a.c, q), w = bm32(v[k1], t.x, t.y, q);
                 v[k0] = add32(u, w);
                 v[k1] = sub32(u, w);
@@ -741,7 +770,7 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
             // inverse GS layer S (ntt_r2_int32_kernels.cc:305-336)
             const int k1 = k0 | (1 << KB);
             const int blk = ((HIB ? (hi << L) : 0) | posmap<LO, EL>(g, k0)) >> (B + 1);
-            const int2 t = __ldg(&a.tab[blk]);
+            const int2 t = NV > 0 ? tv[k0 >> (B + 1)] : __ldg(&a.tab[blk]);
             const int s = add32(v[k0], v[k1]), d = sub32(v[k0], v[k1]);
             v[k0] = br32(s, a.c, q);
             v[k1] = bm32(d, t.x, t.y, q);
@@ -1051,22 +1080,9 @@ __device__ __forceinline__ void k_ntt_body(const KArgs& a) {
     if (active) store_poly<I32, L, EL, LOZ>(v, a, poly, g);
 }
 
-// Two entry points over the same body.  Capping the int32 and radix-4 designs
-// at two resident 256-thread CTAs per SM (128 registers) raised their
-// throughput by up to a fifth on GB300; the same hint made the radix-2 and
-// radix-8 int16 code a fifth slower, so those keep the compiler's default.
-__host__ __device__ constexpr bool kntt_two_ctas(int fam, int threads) {
-    return threads <= 256 && !fam_canon(fam) && (fam_i32(fam) || fam == F_R4F16);
-}
-
-template <int FAM, int L, int EL, int P, bool BR>
-__global__ void __launch_bounds__(P << (L - EL)) k_ntt(const __grid_constant__ KArgs a) {
-    grid_dep_start();
-    k_ntt_body<FAM, L, EL, P, BR>(a);
-}
-
-template <int FAM, int L, int EL, int P, bool BR>
-__global__ void __launch_bounds__(P << (L - EL), 2) k_ntt2(const __grid_constant__ KArgs a) {
+// MB: resident CTAs per SM the registers are budgeted for (kntt_min_blocks)
+template <int FAM, int L, int EL, int P, bool BR, int MB>
+__global__ void __launch_bounds__(P << (L - EL), MB) k_ntt(const __grid_constant__ KArgs a) {
     grid_dep_start();
     k_ntt_body<FAM, L, EL, P, BR>(a);
 }
@@ -1079,22 +1095,38 @@ struct KernelInfo {
     int el = 0;
 };
 
-// elements per thread (log2) and polynomials per CTA of each design
-// Measured on GB300 (one box, same call): 16 coefficients per thread beat 32
-// and 64 for radix-2 int16 forward, radix-4, radix-8 and int32 up to n = 4096
-// (int32 n = 4096: 0.30 vs 0.43 vs 0.49 ms); 32 won for the radix-2 int16
-// inverse at n = 1024 and for int32 n = 2^14 (0.44 vs 0.50 vs 0.54 ms).  At
-// most 1024 threads per polynomial.
+// Shape of a throughput launch, from sweeps of width, CTA size and register
+// budget on 2^26 coefficients (TB/s read and written, one box):
+//   * 16 coefficients per thread: with 32 int32 n = 4096 forward runs at 2.85
+//     for 3.05, radix-4 n = 1024 at 1.84 for 1.98, radix-8 n = 1024 at 1.68 for
+//     1.80.  32 for the radix-2 int16 inverse from n = 2^9 (n = 1024: 2.25 for
+//     2.04), the canonical int16 inverse at 2^12 (2.25 for 2.18) and where 16
+//     would need more than 1024 threads or, at n = 2^13, 512 (lanes 1.83 for
+//     1.75);
+//   * 128-thread CTAs where a polynomial needs no more: an exchange then waits
+//     for four warps, not eight (canonical int32 n = 2048 forward 3.49 for
+//     3.05, lanes 2.49 for 2.45, radix-4 n = 1024 1.98 for 1.95);
+//   * 48 registers a thread at 16 coefficients, 64 to 72 at 32: left to the
+//     compiler, the code takes 56 to 104 and half the warps fit (radix-2 int16
+//     n = 4096 forward 1.27 for 1.66, int32 n = 2048 lanes 1.90 for 2.49).
 __host__ __device__ constexpr int choose_el(int fam, int L) {
     if (L <= 5) return L;
-    if (fam == F_R2I16) return L <= 12 ? (L + 1) / 2 : 6;
-    if (fam_i32(fam)) return L <= 12 ? 4 : (L - 10 > 5 ? L - 10 : 5);
-    return 4;
+    if (fam == F_R2I16) return L >= 9 ? 5 : 4;
+    if (fam == F_C16I && L == 12) return 5;
+    return L == 13 || L == 15 ? 5 : 4;
 }
 __host__ __device__ constexpr int choose_polys(int fam, int L) {
     const int G = 1 << (L - choose_el(fam, L));
-    const int p = 256 / G;
+    const int p = 128 / G;
     return p < 1 ? 1 : p;
+}
+__host__ __device__ constexpr int kntt_min_blocks(int fam, int threads, int el) {
+    if (el >= 5) return threads <= 128 ? 7 : threads <= 256 ? 4 : threads <= 512 ? 2 : 1;
+    if (threads <= 128) return 10;
+    // n = 4096: 40 registers for the radix-4, canonical int16 and canonical
+    // int32 inverse code (1.69 for 1.62, 2.01 for 1.98, 3.69 for 3.58)
+    if (threads <= 256) return fam == F_R4F16 || fam == F_C16F || fam == F_C16I || fam == F_C32I ? 6 : 5;
+    return 2;
 }
 
 // The latency form of a per-plan launch (a launch of at most one CTA per SM):
@@ -1117,10 +1149,8 @@ KernelInfo make_kernel_info() {
     constexpr int EL = LAT ? lat_el(FAM, L) : choose_el(FAM, L);
     constexpr int P = LAT ? 1 : choose_polys(FAM, L);
     KernelInfo ki;
-    if constexpr (kntt_two_ctas(FAM, P << (L - EL)))
-        ki.fn = reinterpret_cast<const void*>(&k_ntt2<FAM, L, EL, P, BR>);
-    else
-        ki.fn = reinterpret_cast<const void*>(&k_ntt<FAM, L, EL, P, BR>);
+    constexpr int MB = LAT ? 1 : kntt_min_blocks(FAM, P << (L - EL), EL);
+    ki.fn = reinterpret_cast<const void*>(&k_ntt<FAM, L, EL, P, BR, MB>);
     ki.threads = P << (L - EL);
     ki.smem = num_windows(FAM, L, EL) > 1 ? P * xwords(L) * 4 : 0;
     ki.polys = P;
