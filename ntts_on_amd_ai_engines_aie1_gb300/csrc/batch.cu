@@ -27,7 +27,8 @@ struct gbntt_batch {
         std::vector<SegDev> live;       // zero-copy layout: the descriptors d_segs holds now
         long long total_tiles = 0;
         int stage_bytes = 0, smem = 0, grid = 0;
-        float ms = -1.f;                // autotuner timing
+        float ms = -1.f;                // autotuner timing: cold + warm
+        float cold = -1.f, warm = -1.f;
     };
     struct Pending {                    // a batched segment before the layouts are built
         int k, fam, L, eb;
@@ -39,6 +40,7 @@ struct gbntt_batch {
         std::vector<Pending> pending;
         std::vector<Layout> layouts;    // candidate configurations
         int chosen = 0;
+        int staged = 0;                 // the fastest staged layout
         std::vector<int> user_index;    // caller's segment of each SegDev
         Layout zlay;                    // zero-copy launch (k_batch_zc), when a configuration has one
     };
@@ -86,16 +88,21 @@ int launch_layout(gbntt_batch* b, int pi, const gbntt_batch::Layout& lay, cudaSt
     bd.wait_polls = batch_wait_polls();
     int sb = lay.stage_bytes;
     void* args[] = {&bd, &sb};
-    cudaError_t e = cudaLaunchKernel(lay.cfg.fn, dim3(lay.grid), dim3(lay.cfg.cta), args, lay.smem, s);
+    // the staged kernel owns counters that its last CTA resets, so its launches
+    // are plain; the others are programmatic dependent launches (grid_dep_start)
+    cudaError_t e = launch_kernel(lay.cfg.fn, (unsigned)lay.grid, lay.cfg.cta, lay.smem, args, s,
+                                  lay.cfg.form != BF_STAGED);
     if (e != cudaSuccess) return batch_fail(GBNTT_ERR_CUDA, std::string("batch launch: ") + cudaGetErrorString(e));
     gbntt_internal_count_launch();
     return GBNTT_OK;
 }
 
 int launch_batch(gbntt_batch* b, cudaStream_t s) {
+    // a poll limit of the caller's own asks for the kernel that has waits
+    const bool staged = batch_wait_polls() != BATCH_WAIT_POLLS;
     for (int i = 0; i < b->nparts; ++i) {
         auto& p = b->parts[i];
-        const int rc = launch_layout(b, i, p.layouts[p.chosen], s);
+        const int rc = launch_layout(b, i, p.layouts[staged ? p.staged : p.chosen], s);
         if (rc != GBNTT_OK) return rc;
     }
     for (size_t k = 0; k < b->user.size(); ++k) {
@@ -109,19 +116,15 @@ int launch_batch(gbntt_batch* b, cudaStream_t s) {
 
 // Times every candidate configuration of every part on the batch itself (the
 // outputs it writes are the batch's own results) and keeps the fastest.
-// A batch whose inputs and outputs fit in L2 would be timed from L2 if its
-// launches ran back to back, which is not how it meets its data in use: each
-// of its timed launches then follows a write of a buffer twice the L2 size.
-// (On a ragged radix-8 batch of 13 MB, back-to-back timing chose 32
-// coefficients per thread, 18.8 against 20.2 us; from HBM the choice it
-// missed runs 27.9 against 35.3 us.)
+// A batch whose inputs and outputs fit in L2 is timed from HBM too, each such
+// launch after a write of a buffer twice the L2 size: back to back its launches
+// would only ever find their data in L2.  (On a ragged radix-8 batch of 13 MB,
+// back-to-back timing alone chose 32 coefficients per thread, 18.8 against
+// 20.2 us; from HBM the choice it missed runs 27.9 against 35.3 us.)
 int autotune(gbntt_batch* b) {
     cudaStream_t s;
     if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess)
         return batch_fail(GBNTT_ERR_CUDA, "autotune stream");
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
     size_t footprint = 0;
     for (const auto& u : b->user) {
         int64_t n = 0, eb = 0;
@@ -144,66 +147,77 @@ int autotune(gbntt_batch* b) {
         if (p.layouts.size() < 2) continue;
         for (size_t c = 0; c < p.layouts.size() && rc == GBNTT_OK; ++c)
             for (int w = 0; w < 2 && rc == GBNTT_OK; ++w) rc = launch_layout(b, i, p.layouts[c], s);
-        // five interleaved rounds, best round per configuration (clock drift
+        // Five interleaved rounds, the best time per configuration (clock drift
         // hits all alike; configurations 3 % apart were ranked inconsistently
-        // with three)
+        // with three).  A round enqueues, per configuration, a launch after the
+        // fill (only for a batch that fits in L2) and three back to back timed
+        // as one, then waits once: the launches meet the GPU as timed steps do
+        // (the next one queued while the fill runs), not after an idle gap.  A
+        // batch in L2 is met both ways in use, first from HBM and then again
+        // from L2, and the ways rank kernels differently (few large tiles: the
+        // direct kernel 16.4 against 14.4 us from L2 and ahead of the staged
+        // one from HBM), so the sum decides.  Configurations more than 15 %
+        // above the best of the rounds so far sit out.
+        const size_t per = flush ? 2 : 1;              // timed spans of a configuration and round
+        std::vector<cudaEvent_t> ev(2 * per * p.layouts.size());
+        for (auto& x : ev) cudaEventCreate(&x);
         for (int round = 0; round < 5 && rc == GBNTT_OK; ++round) {
-            if (flush) {
-                // every configuration three times, each launch after the fill
-                // and timed alone, the whole round enqueued before one wait:
-                // the launches meet the GPU as timed steps do (the next one
-                // queued while the fill runs), not after an idle gap
-                const size_t nl = p.layouts.size() * 3;
-                std::vector<cudaEvent_t> ev(2 * nl);
-                for (auto& x : ev) cudaEventCreate(&x);
-                for (size_t c = 0; c < p.layouts.size() && rc == GBNTT_OK; ++c)
-                    for (int w = 0; w < 3 && rc == GBNTT_OK; ++w) {
-                        cudaMemsetAsync(flush, w, flush_bytes, s);
-                        cudaEventRecord(ev[2 * (3 * c + w)], s);
-                        rc = launch_layout(b, i, p.layouts[c], s);
-                        cudaEventRecord(ev[2 * (3 * c + w) + 1], s);
-                    }
-                if (rc == GBNTT_OK && cudaStreamSynchronize(s) != cudaSuccess)
-                    rc = batch_fail(GBNTT_ERR_CUDA, "autotune timing");
-                for (size_t c = 0; c < p.layouts.size() && rc == GBNTT_OK; ++c) {
-                    float ms = 0.f;
-                    for (int w = 0; w < 3; ++w) {
-                        float one = 0.f;
-                        cudaEventElapsedTime(&one, ev[2 * (3 * c + w)], ev[2 * (3 * c + w) + 1]);
-                        ms += one / 3.f;
-                    }
-                    if (p.layouts[c].ms < 0.f || ms < p.layouts[c].ms) p.layouts[c].ms = ms;
+            float fastest = -1.f;
+            for (const auto& l : p.layouts)
+                if (l.ms >= 0.f && (fastest < 0.f || l.ms < fastest)) fastest = l.ms;
+            auto runs = [&](size_t c) { return fastest < 0.f || p.layouts[c].ms <= 1.15f * fastest; };
+            for (size_t c = 0; c < p.layouts.size(); ++c) {
+                if (!runs(c)) continue;
+                for (size_t w = 0; w < per && rc == GBNTT_OK; ++w) {
+                    const bool cold = w + 1 < per;
+                    if (cold) cudaMemsetAsync(flush, round, flush_bytes, s);
+                    cudaEventRecord(ev[2 * (per * c + w)], s);
+                    for (int k = 0; k < (cold ? 1 : 3) && rc == GBNTT_OK; ++k) rc = launch_layout(b, i, p.layouts[c], s);
+                    cudaEventRecord(ev[2 * (per * c + w) + 1], s);
                 }
-                for (auto& x : ev) cudaEventDestroy(x);
-                continue;
             }
-            // inputs larger than L2: five launches back to back
+            if (rc == GBNTT_OK && cudaStreamSynchronize(s) != cudaSuccess)
+                rc = batch_fail(GBNTT_ERR_CUDA, "autotune timing");
             for (size_t c = 0; c < p.layouts.size() && rc == GBNTT_OK; ++c) {
-                float ms = 0.f;
-                cudaEventRecord(e0, s);
-                for (int w = 0; w < 5 && rc == GBNTT_OK; ++w) rc = launch_layout(b, i, p.layouts[c], s);
-                cudaEventRecord(e1, s);
-                if (cudaEventSynchronize(e1) != cudaSuccess) rc = batch_fail(GBNTT_ERR_CUDA, "autotune timing");
-                cudaEventElapsedTime(&ms, e0, e1);
-                ms /= 5.f;
-                if (p.layouts[c].ms < 0.f || ms < p.layouts[c].ms) p.layouts[c].ms = ms;
+                auto& l = p.layouts[c];
+                if (!runs(c)) continue;
+                l.ms = 0.f;
+                for (size_t w = 0; w < per; ++w) {
+                    float& least = w + 1 < per ? l.cold : l.warm;
+                    float ms = 0.f;
+                    cudaEventElapsedTime(&ms, ev[2 * (per * c + w)], ev[2 * (per * c + w) + 1]);
+                    if (w + 1 == per) ms /= 3.f;
+                    if (least < 0.f || ms < least) least = ms;
+                    l.ms += least;
+                }
             }
         }
-        size_t best = 0;
-        for (size_t c = 1; c < p.layouts.size(); ++c)
-            if (p.layouts[c].ms >= 0.f && p.layouts[c].ms < p.layouts[best].ms) best = c;
+        for (auto& x : ev) cudaEventDestroy(x);
+        size_t best = 0, staged = p.staged;
+        for (size_t c = 0; c < p.layouts.size(); ++c) {
+            if (p.layouts[c].ms < 0.f) continue;
+            if (p.layouts[c].ms < p.layouts[best].ms) best = c;
+            if (p.layouts[c].cfg.form == BF_STAGED && p.layouts[c].ms < p.layouts[staged].ms) staged = c;
+        }
+        p.staged = (int)staged;
         // GBNTT_TUNE_FORCE="<log2 coefficients per thread>,<CTAs per SM>" pins the
         // choice (the timing launches still run), e.g. to profile the kernel a
         // normal run picks while a profiler slows every launch down; "tc" pins
-        // the tensor-core kernel
+        // the tensor-core kernel, "d<threads per CTA>,<log2 coefficients per
+        // thread>" a direct one
         if (const char* f = std::getenv("GBNTT_TUNE_FORCE")) {
             int el = -1, occ = -1;
             if (std::strcmp(f, "tc") == 0) {
                 for (size_t c = 0; c < p.layouts.size(); ++c)
-                    if (p.layouts[c].cfg.tc) best = c;
+                    if (p.layouts[c].cfg.form == BF_TC) best = c;
+            } else if (std::sscanf(f, "d%d,%d", &el, &occ) == 2) {
+                for (size_t c = 0; c < p.layouts.size(); ++c)
+                    if (p.layouts[c].cfg.form == BF_DIRECT && p.layouts[c].cfg.cta == el && p.layouts[c].cfg.elmax == occ)
+                        best = c;
             } else if (std::sscanf(f, "%d,%d", &el, &occ) == 2)
                 for (size_t c = 0; c < p.layouts.size(); ++c)
-                    if (!p.layouts[c].cfg.tc && p.layouts[c].cfg.elmax == el && p.layouts[c].cfg.occ == occ) {
+                    if (p.layouts[c].cfg.form == BF_STAGED && p.layouts[c].cfg.elmax == el &&
+                        p.layouts[c].cfg.occ == occ) {
                         best = c;
                         break;
                     }
@@ -214,12 +228,11 @@ int autotune(gbntt_batch* b) {
                 std::fprintf(stderr, "gbntt autotune: %s part, %d coefficients/thread, %d threads/CTA, %d CTAs/SM, "
                              "families 0x%x%s: %.2f us%s\n", p.i32 ? "int32" : "int16", 1 << p.layouts[c].cfg.elmax,
                              p.layouts[c].cfg.cta, p.layouts[c].cfg.occ, p.layouts[c].cfg.set,
-                             p.layouts[c].cfg.tc ? ", tensor cores" : "",
+                             p.layouts[c].cfg.form == BF_TC ? ", tensor cores"
+                             : p.layouts[c].cfg.form == BF_DIRECT ? ", direct" : "",
                              1e3 * p.layouts[c].ms, c == best ? "  <- chosen" : "");
     }
     if (flush) cudaFree(flush);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     cudaStreamDestroy(s);
     return rc;
 }
@@ -381,7 +394,8 @@ int gbntt_batch_create(gbntt_batch** out, const gbntt_segment* segs, uint32_t ns
         const BatchConfig* cfgs = nullptr;
         const int ncfg = part.i32 ? batch_configs_i32(&cfgs) : batch_configs_i16(&cfgs);
         auto covers = [&](const BatchConfig& c) {
-            return (c.set & part.fam_mask) == part.fam_mask && (c.tc ? tc : config_fits(c, maxL));
+            return (c.set & part.fam_mask) == part.fam_mask &&
+                   (c.form == BF_TC ? tc : batch_fits(maxL, c.cta, c.elmax));
         };
         for (int c = 0; c < ncfg; ++c)
             if (covers(cfgs[c])) {
@@ -393,7 +407,19 @@ int gbntt_batch_create(gbntt_batch** out, const gbntt_segment* segs, uint32_t ns
             gbntt_batch_destroy(b);
             return batch_fail(GBNTT_ERR_ARG, "no persistent kernel covers these designs");
         }
-        if (flags & GBNTT_BATCH_NO_TUNE) part.layouts.resize(1);   // the first (widest, most specific) one
+        // untuned: the first (tensor-core, else the widest, most specific) one,
+        // and the first staged one
+        auto first_staged = [&] {
+            size_t c = 0;
+            while (part.layouts[c].cfg.form != BF_STAGED) ++c;   // every family has a staged kernel
+            return c;
+        };
+        if (flags & GBNTT_BATCH_NO_TUNE) {
+            const size_t c = first_staged();
+            if (c > 1) std::swap(part.layouts[1], part.layouts[c]);
+            part.layouts.resize(c ? 2 : 1);
+        }
+        part.staged = (int)first_staged();
         // zero copy: the narrowest covering configuration
         for (int c = 0; c < ncfg; ++c)
             if (cfgs[c].zfn && covers(cfgs[c]) && (!part.zlay.cfg.zfn || cfgs[c].elmax < part.zlay.cfg.elmax))
@@ -420,14 +446,15 @@ int gbntt_batch_create(gbntt_batch** out, const gbntt_segment* segs, uint32_t ns
             sd.n = 1 << L;
             sd.elem_bytes = eb;
             sd.variant = variant_id(fam, L);
-            sd.polys_per_tile = lay.cfg.tc ? TC_TILE >> L : lay.cfg.cta >> (L - batch_el(L, elmax));
+            const int unit = lay.cfg.form == BF_DIRECT ? direct_unit(lay.cfg.cta) : lay.cfg.cta;   // threads a tile stands for
+            sd.polys_per_tile = lay.cfg.form == BF_TC ? TC_TILE >> L : unit >> (L - batch_el(L, elmax));
             sd.tiles = ((long long)u.count + sd.polys_per_tile - 1) / sd.polys_per_tile;
             sd.tile0 = lay.total_tiles;
             lay.total_tiles += sd.tiles;
-            if (!lay.cfg.tc) {
+            if (lay.cfg.form == BF_STAGED)
                 lay.stage_bytes = std::max(lay.stage_bytes, batch_stage_bytes(lay.cfg.cta, L, eb, elmax));
+            if (lay.cfg.form != BF_TC)
                 lay.smem = std::max(lay.smem, batch_xbuf_bytes(lay.cfg.cta, L, elmax));
-            }
             lay.segs.push_back(sd);
         }
       }
@@ -443,7 +470,7 @@ int gbntt_batch_create(gbntt_batch** out, const gbntt_segment* segs, uint32_t ns
             gbntt_batch::Layout& lay = *lp;
             const bool zc = (lp == &b->parts[i].zlay);     // one staging buffer instead of two
             lay.stage_bytes = (lay.stage_bytes + 127) & ~127;
-            if (!lay.cfg.tc) lay.smem = SMEM_HEADER + (zc ? 1 : 2) * lay.stage_bytes + lay.smem;
+            if (lay.cfg.form == BF_STAGED) lay.smem = SMEM_HEADER + (zc ? 1 : 2) * lay.stage_bytes + lay.smem;
             const void* fn = zc ? lay.cfg.zfn : lay.cfg.fn;
             cudaError_t e = raise_smem_limit(fn, lay.smem);
             int per_sm = 0;
@@ -457,7 +484,8 @@ int gbntt_batch_create(gbntt_batch** out, const gbntt_segment* segs, uint32_t ns
             // write-only end of the launch (benchmark batch end to end: 1, 2, 3,
             // 4 CTAs/SM -> 100, 106, 103, 100 M NTT/s on one box).
             const int resident = zc ? std::min(per_sm, 2) : per_sm;
-            lay.grid = (int)std::min<long long>((long long)resident * sms, lay.total_tiles);
+            lay.grid = lay.cfg.form == BF_DIRECT ? (int)(lay.total_tiles * (direct_unit(lay.cfg.cta) / lay.cfg.cta))
+                                                 : (int)std::min<long long>((long long)resident * sms, lay.total_tiles);
             e = cudaMalloc(&lay.d_segs, sizeof(SegDev) * lay.segs.size());
             if (e == cudaSuccess)
                 e = cudaMemcpy(lay.d_segs, lay.segs.data(), sizeof(SegDev) * lay.segs.size(), cudaMemcpyHostToDevice);

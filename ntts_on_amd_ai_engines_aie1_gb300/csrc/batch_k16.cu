@@ -17,6 +17,7 @@ const void* batch_kernels_c16(int el, int set, int occ);
 const void* batch_kernels_c16_small(int el, int set, int occ, int cta);
 const void* batch_zc_kernel_c16(int set, int el);
 const void* batch_kernel_tc16();
+const void* batch_direct_i16(int el, int set, int occ, int cta);
 
 namespace {
 constexpr int R2 = (1 << F_R2F16) | (1 << F_R2I16);
@@ -28,7 +29,7 @@ constexpr int C16 = (1 << F_C16F) | (1 << F_C16I);   // canonical forward + inve
 struct Key {
     int el, set, occ;
     int cta = BATCH_CTA;
-    bool tc = false;
+    int form = BF_STAGED;
 };
 // 256-thread CTAs with 64, 32 or 16 coefficients per thread; the narrower
 // ones carry less unrolled code per variant and fit more CTAs per SM (occ:
@@ -39,7 +40,7 @@ constexpr Key kKeys[] = {
     {6, R4, 0}, {5, R4, 0}, {6, R2, 0}, {5, R2, 0}, {6, R8, 0}, {5, R8, 0}, {5, ALL16, 0},
     {4, R4, 0}, {4, R4, 5}, {4, R4, 6}, {4, R2, 0}, {4, R2, 5}, {4, R8, 0}, {4, R8, 5}, {4, ALL16, 0},
     // canonical families on the tensor cores (n = 2^5 .. 2^10)
-    {5, C16, TC_OCC, TC_CTA, true},
+    {5, C16, TC_OCC, TC_CTA, BF_TC},
     // canonical families: 16 coefficients per thread at 4, 5 and 6 CTAs/SM, 32 at 3
     // and 4 (8 per thread at 8 CTAs/SM spilled at its 32-register budget)
     {4, C16, 6}, {4, C16, 5}, {4, C16, 0}, {5, C16, 0}, {5, C16, 4},
@@ -49,6 +50,9 @@ constexpr Key kKeys[] = {
     // 32 coefficients per thread in 64-thread CTAs (n <= 2^11): one warp per
     // 1024-point polynomial (the fastest on batches of 4x the benchmark's)
     {5, C16, 12, 64},
+    // straight from and to global memory
+    {4, R4, 10, 128, BF_DIRECT}, {4, R4, 6, 256, BF_DIRECT}, {4, R2, 10, 128, BF_DIRECT}, {4, R2, 5, 256, BF_DIRECT},
+    {4, R8, 10, 128, BF_DIRECT}, {4, R8, 5, 256, BF_DIRECT}, {4, C16, 10, 128, BF_DIRECT}, {4, C16, 6, 256, BF_DIRECT},
 };
 constexpr int kN = (int)(sizeof(kKeys) / sizeof(kKeys[0]));
 BatchConfig kI16[kN];
@@ -59,8 +63,10 @@ int batch_configs_i16(const BatchConfig** out) {
         for (int i = 0; i < kN; ++i) {
             const Key k = kKeys[i];
             const void* fn = nullptr;
-            if (k.tc) {
+            if (k.form == BF_TC) {
                 fn = batch_kernel_tc16();
+            } else if (k.form == BF_DIRECT) {
+                fn = batch_direct_i16(k.el, k.set, k.occ, k.cta);
             } else if (k.cta != BATCH_CTA) {
                 fn = batch_kernels_c16_small(k.el, k.set, k.occ, k.cta);
             } else {
@@ -68,10 +74,10 @@ int batch_configs_i16(const BatchConfig** out) {
                                  batch_kernels_i16_w16, batch_kernels_i16_w16g, batch_kernels_c16})
                     if (!fn) fn = get(k.el, k.set, k.occ);
             }
-            const void* zfn = k.tc || k.cta != BATCH_CTA ? nullptr
+            const void* zfn = k.form != BF_STAGED || k.cta != BATCH_CTA ? nullptr
                               : k.set == C16 ? (k.occ == 0 ? batch_zc_kernel_c16(k.set, k.el) : nullptr)
                                              : batch_zc_kernel_i16(k.set, k.el);
-            kI16[i] = BatchConfig{false, k.el, k.set, fn, zfn, k.cta, k.occ, k.tc};
+            kI16[i] = BatchConfig{false, k.el, k.set, fn, zfn, k.cta, k.occ, k.form};
         }
         return true;
     }();

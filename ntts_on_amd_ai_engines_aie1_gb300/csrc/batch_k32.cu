@@ -7,11 +7,13 @@ namespace gbntt {
 
 const void* batch_kernels_i32_w16(int occ, bool zero_copy);
 const void* batch_kernels_c32(int el, int occ, bool zero_copy);
+const void* batch_direct_i32(int el, int set, int occ, int cta);
 
 namespace {
 constexpr int I32SET = (1 << F_R2F32) | (1 << F_R2G32);
 constexpr int C32 = (1 << F_C32F) | (1 << F_C32I);   // canonical forward + inverse
-BatchConfig kI32[6];
+constexpr int kN = 14;
+BatchConfig kI32[kN];
 }  // namespace
 
 int batch_configs_i32(const BatchConfig** out) {
@@ -26,11 +28,19 @@ int batch_configs_i32(const BatchConfig** out) {
         kI32[4] = BatchConfig{true, 4, C32, batch_kernels_c32(4, 0, false), batch_kernels_c32(4, 0, true),
                               BATCH_CTA, 0};
         kI32[5] = BatchConfig{true, 4, C32, batch_kernels_c32(4, 4, false), nullptr, BATCH_CTA, 4};
+        // straight from and to global memory
+        int i = 6;
+        for (const int set : {I32SET, C32}) {
+            kI32[i++] = BatchConfig{true, 4, set, batch_direct_i32(4, set, 10, 128), nullptr, 128, 10, BF_DIRECT};
+            kI32[i++] = BatchConfig{true, 4, set, batch_direct_i32(4, set, 5, 256), nullptr, 256, 5, BF_DIRECT};
+            kI32[i++] = BatchConfig{true, 5, set, batch_direct_i32(5, set, 4, 256), nullptr, 256, 4, BF_DIRECT};
+            kI32[i++] = BatchConfig{true, 4, set, batch_direct_i32(4, set, 2, 512), nullptr, 512, 2, BF_DIRECT};
+        }
         return true;
     }();
     (void)built;
     *out = kI32;
-    return 6;
+    return kN;
 }
 
 }  // namespace gbntt

@@ -283,7 +283,14 @@ inline bool variant_supported(int fam, int L) {
 }
 
 
-// one compiled configuration of the persistent kernel
+// the kernels a batch part can run on: k_batch (staged, persistent, bounded
+// waits), the tensor-core kernel (tc16.cuh) and k_batch_direct (batch_direct.cuh)
+enum { BF_STAGED = 0, BF_TC = 1, BF_DIRECT = 2 };
+
+// threads whose polynomials make a tile of the direct kernel
+__host__ __device__ constexpr int direct_unit(int cta) { return cta > BATCH_CTA ? cta : BATCH_CTA; }
+
+// one compiled configuration of a batch kernel
 struct BatchConfig {
     bool i32;
     int elmax;   // log2 coefficients per thread
@@ -292,12 +299,11 @@ struct BatchConfig {
     const void* zfn;   // zero-copy form (k_batch_zc), or nullptr
     int cta;           // threads per CTA
     int occ;           // resident CTAs per SM the registers are budgeted for (0: the default)
-    bool tc = false;   // the tensor-core kernel (tc16.cuh): its own tile size, no shared memory
+    int form = BF_STAGED;
 };
 
-// the window/exchange configuration carries a transform of 2^L coefficients
-// (never true of the tensor-core one: batch.cu asks tc_supported)
-inline bool config_fits(const BatchConfig& c, int L) { return !c.tc && batch_fits(L, c.cta, c.elmax); }
+// the staged configuration carries a transform of 2^L coefficients
+inline bool config_fits(const BatchConfig& c, int L) { return c.form == BF_STAGED && batch_fits(L, c.cta, c.elmax); }
 
 // the persistent launch of a batch part: storage type and arithmetic
 // (the reference's lanes or the canonical families) -- 4 parts

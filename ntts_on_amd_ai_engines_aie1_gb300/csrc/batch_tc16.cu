@@ -15,6 +15,7 @@ __global__ void __launch_bounds__(TC_CTA, TC_OCC) k_batch_tc16(const BatchDev b,
     __shared__ __align__(128) unsigned char rings[TC_CTA / 32][TC_WARP_RING];
     unsigned char* ring = rings[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
+    grid_dep_start();
     const long long warps = (long long)gridDim.x * (TC_CTA / 32);
     long long t = (long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
     int s = 0;

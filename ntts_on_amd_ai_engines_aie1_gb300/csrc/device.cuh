@@ -1024,30 +1024,21 @@ __device__ __forceinline__ void store_poly(int (&v)[1 << EL], const KArgs& a, lo
 // the transform kernel: P polynomials per CTA, G = 2^(L-EL) threads each
 // ---------------------------------------------------------------------------
 
+// one CTA's P polynomials, poly0 the first: global memory to global memory
 template <int FAM, int L, int EL, int P, bool BR>
-__device__ __forceinline__ void k_ntt_body(const KArgs& a) {
+__device__ __forceinline__ void ntt_tile(const KArgs& a, int lean, long long poly0, int* smem) {
     constexpr int G = 1 << (L - EL);
     constexpr int NS = nsteps(FAM, L);
-    constexpr int N = 1 << L;
     constexpr int SW = xwords(L);
     constexpr bool I32 = fam_i32(FAM);
-    extern __shared__ int smem[];
     const int tid = threadIdx.x;
     const int lp = tid / G, g = tid % G;
-    const long long poly = (long long)blockIdx.x * P + lp;
+    const long long poly = poly0 + lp;
     const bool active = poly < a.batch;
     int* sp = smem + lp * SW;
     int v[1 << EL];
     constexpr int LO0 = window_lo(FAM, L, EL, 0);
     constexpr int LOZ = window_lo(FAM, L, EL, NS - 1);
-    // Every stage's table loads sit on the transform's dependent path; in a
-    // launch of a few polynomials (latency) they would wait stage by stage, so
-    // the host asks for the whole table in L1 first, beside the polynomial's load.
-    {
-        const char* tb = a.tab16 ? reinterpret_cast<const char*>(a.tab16) : reinterpret_cast<const char*>(a.tab);
-        for (int off = tid * 128; off < a.tab_bytes; off += (int)blockDim.x * 128)
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(tb + off));
-    }
     if (active) {
         load_poly<I32, L, EL, LO0>(v, a, poly, g);
     } else {
@@ -1070,7 +1061,7 @@ __device__ __forceinline__ void k_ntt_body(const KArgs& a) {
     }
     prologue<FAM>(v, a);
     const KC kc = make_kc(a);
-    run_steps<FAM, L, EL>(v, sp, g, kc, a.lean, fresh, std::make_integer_sequence<int, NS>{});
+    run_steps<FAM, L, EL>(v, sp, g, kc, lean, fresh, std::make_integer_sequence<int, NS>{});
     epilogue<FAM, BR>(v, a);
     if constexpr (BR) {
         permute_br<L, EL, LOZ>(v, sp, g);
@@ -1078,6 +1069,18 @@ __device__ __forceinline__ void k_ntt_body(const KArgs& a) {
         if (a.natural_out) permute_br<L, EL, LOZ>(v, sp, g);
     }
     if (active) store_poly<I32, L, EL, LOZ>(v, a, poly, g);
+}
+
+template <int FAM, int L, int EL, int P, bool BR>
+__device__ __forceinline__ void k_ntt_body(const KArgs& a) {
+    extern __shared__ int smem[];
+    // Every stage's table loads sit on the transform's dependent path; in a
+    // launch of a few polynomials (latency) they would wait stage by stage, so
+    // the host asks for the whole table in L1 first, beside the polynomial's load.
+    const char* tb = a.tab16 ? reinterpret_cast<const char*>(a.tab16) : reinterpret_cast<const char*>(a.tab);
+    for (int off = (int)threadIdx.x * 128; off < a.tab_bytes; off += (int)blockDim.x * 128)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(tb + off));
+    ntt_tile<FAM, L, EL, P, BR>(a, a.lean, (long long)blockIdx.x * P, smem);
 }
 
 // MB: resident CTAs per SM the registers are budgeted for (kntt_min_blocks)

@@ -23,9 +23,9 @@ uint32_t f16_bits(int v) {
 struct Limbs {
     uint32_t h, l;
 };
-Limbs limbs(int64_t w, int64_t q, int hs) {
-    int v = (int)(w > q / 2 ? w - q : w);
-    int l = ((v % 256) + 256) % 256;
+Limbs limbs(uint32_t w, uint32_t q, int hs) {
+    const int v = w > q / 2 ? (int)w - (int)q : (int)w;
+    int l = v & 255;
     if (l >= 128) l -= 256;
     return {f16_bits(hs * ((v - l) / 256)), f16_bits(2 * l)};
 }
@@ -79,7 +79,7 @@ bool tc_supported(int L, int64_t q) {
     return 2 * (d + 32) < q;
 }
 
-void tc_build(int L, int64_t q, int64_t root, bool inverse, bool natural, bool scale, std::vector<uint32_t>& out,
+void tc_build(int L, int64_t modulus, int64_t root, bool inverse, bool natural, bool scale, std::vector<uint32_t>& out,
               uint32_t* ke, uint32_t* corr) {
     Maps M;
     M.LK = tc_lk(L);
@@ -89,13 +89,14 @@ void tc_build(int L, int64_t q, int64_t root, bool inverse, bool natural, bool s
     M.lb = inverse && !natural;
     M.sb = !inverse && !natural;
     const int S1 = tc_s1(M.LK), S2 = tc_s2(M.LK), NT = tc_cols(M.LK) / 8;
-    const int64_t n = (int64_t)1 << L;
-    const int64_t w0 = inverse ? modinv(root, q) : root;
-    std::vector<int64_t> pw(n);                       // powers of the root
+    // q < 2^15: every product below fits 32 bits
+    const uint32_t n = 1u << L, q = (uint32_t)modulus;
+    const uint32_t w0 = (uint32_t)(inverse ? modinv(root, modulus) : root);
+    std::vector<uint32_t> pw(n);                      // powers of the root
     pw[0] = 1 % q;
-    for (int64_t i = 1; i < n; ++i) pw[i] = pw[i - 1] * w0 % q;
-    auto power = [&](int64_t e) { return pw[e & (n - 1)]; };
-    const int64_t fac = scale ? modinv(n % q, q) : 1;
+    for (uint32_t i = 1; i < n; ++i) pw[i] = pw[i - 1] * w0 % q;
+    auto power = [&](int e) { return pw[(uint32_t)e & (n - 1)]; };
+    const uint32_t fac = scale ? (uint32_t)modinv(n % q, modulus) : 1u;
     out.assign((size_t)tc_words(M.LK) * 4, 0);
     uint32_t* A = out.data();
     uint32_t* B = A + (size_t)tc_a_words(M.LK) * 4;
@@ -108,7 +109,7 @@ void tc_build(int L, int64_t q, int64_t root, bool inverse, bool natural, bool s
                 const int row = g + 8 * (r & 1), k0 = 2 * t + 8 * (r >> 1);
                 Limbs hi[2], lo[2];
                 for (int e = 0; e < 2; ++e) {
-                    const int64_t w = power((int64_t)M.m(row) * M.u(s, k0 + e) * M.R2);
+                    const uint32_t w = power(M.m(row) * M.u(s, k0 + e) * M.R2);
                     hi[e] = limbs(w * 256 % q, q, 2);
                     lo[e] = limbs(w, q, 2);
                 }
@@ -127,7 +128,7 @@ void tc_build(int L, int64_t q, int64_t root, bool inverse, bool natural, bool s
                         const int k = 2 * t + 8 * r + e;
                         int pc, c;
                         M.col(2 * s + (k >> 3), k & 7, &pc, &c);
-                        const int64_t w = pc == po ? power((int64_t)c * v * M.R1) : 0;
+                        const uint32_t w = pc == po ? power(c * v * M.R1) : 0u;
                         hi[e] = limbs(w * 256 % q, q, 512);
                         lo[e] = limbs(w, q, 512);
                     }
@@ -145,15 +146,16 @@ void tc_build(int L, int64_t q, int64_t root, bool inverse, bool natural, bool s
                 for (int i = 0; i < 4; ++i) {
                     int po, c;
                     M.col(j, 2 * t + (i & 1), &po, &c);
-                    const int64_t m = M.m(g + 8 * (i >> 1)) + 16 * p;
-                    const int64_t w = power(m * c) * fac % q;
+                    const int m = M.m(g + 8 * (i >> 1)) + 16 * p;
+                    const uint32_t w = power(m * c) * fac % q;
                     uint32_t* d = W + (((j * S1 + p) * 2 + (i >> 1)) * 32 + lane) * 4 + 2 * (i & 1);
-                    d[0] = (uint32_t)w;
-                    d[1] = (uint32_t)(((uint64_t)w << 32) / (uint64_t)q);
+                    const uint32_t hi = (w << 16) / q;
+                    d[0] = w;
+                    d[1] = hi << 16 | ((w << 16) % q << 16) / q;      // floor(w 2^32 / q)
                 }
     }
-    *ke = (uint32_t)((((int64_t)1 << 28) / q) * q);
-    *corr = (uint32_t)((q - (int64_t)32768 * 16 % q) % q);
+    *ke = ((1u << 28) / q) * q;
+    *corr = (q - (32768u * 16) % q) % q;
 }
 
 }  // namespace gbntt
