@@ -147,9 +147,10 @@ __host__ __device__ __forceinline__ int rsz32(int a, int b) {
     return (int)(((long long)a * b + (long long)(unsigned long long)bias) >> 32);
 }
 
-// round(p / 2^31), ties toward zero
-__device__ __forceinline__ int rsz31(long long p) {
-    return (int)((p + 0x3FFFFFFFLL + (long long)((unsigned long long)p >> 63)) >> 31);
+// round(a b / 2^31), ties toward zero (bias and sign as in rsz32)
+__host__ __device__ __forceinline__ int rsz31(int a, int b) {
+    const unsigned bias = 0x3FFFFFFFu + ((unsigned)(a ^ b) >> 31);
+    return (int)(((long long)a * b + (long long)(unsigned long long)bias) >> 31);
 }
 
 __device__ __forceinline__ int wrap16(int x) { return (int)(short)x; }
@@ -204,10 +205,10 @@ __device__ __forceinline__ int add32(int a, int b) { return (int)((unsigned)a + 
 __device__ __forceinline__ int sub32(int a, int b) { return (int)((unsigned)a - (unsigned)b); }
 
 // radix-8 reduction tile: m' = round(y w' / 2^31) truncated to int16, then
-// y w - m' q kept as int16 (ntt_r8_kernels.cc:30-177)
+// y w - m' q kept as int16 (ntt_r8_kernels.cc:30-177).  The truncation of m'
+// changes m' q by a multiple of 2^16, which the last one drops, so it is left out.
 __device__ __forceinline__ int r8red(int y, int tw, int wq, int q) {
-    const int m16 = (int)(short)rsz31((long long)y * wq);
-    return wrap16((int)((unsigned)y * (unsigned)tw - (unsigned)m16 * (unsigned)q));
+    return wrap16((int)((unsigned)y * (unsigned)tw - (unsigned)rsz31(y, wq) * (unsigned)q));
 }
 
 // Full Barrett multiplication by a constant, fully reduced
@@ -296,10 +297,9 @@ template <bool SCALE, int E>
 __device__ __forceinline__ void epilogue_all(int (&v)[E], const KArgs& a);
 
 // Canonical families: every lane to [0, q), or n^-1 times it (a Shoup
-// multiplication, [0, 2q), then one subtraction) for a scaled inverse.  (int32
-// lanes end below 4q, so two subtract-and-minimum steps would reduce them
-// without a multiply; measured mixed against the Barrett step, -4 % to +12 %
-// per design, so every family keeps the Barrett step.)
+// multiplication, [0, 2q), then one subtraction) for a scaled inverse.  int32
+// lanes end below 4q: two add-and-minimum steps.  int16 lanes end below 2^29: a
+// Barrett step and one subtraction.
 template <bool I32, int E>
 __device__ __forceinline__ void epilogue_canon(int (&v)[E], const KArgs& a, bool scale) {
     const unsigned q = (unsigned)a.q;
@@ -307,6 +307,10 @@ __device__ __forceinline__ void epilogue_canon(int (&v)[E], const KArgs& a, bool
         const unsigned w = a.ninv, wq = a.ninv_q;
 #pragma unroll
         for (int k = 0; k < E; ++k) v[k] = (int)lazy_sub(shoup_mul((unsigned)v[k], w, wq, q), q);
+    } else if constexpr (I32) {
+        const unsigned q2 = (unsigned)a.c;
+#pragma unroll
+        for (int k = 0; k < E; ++k) v[k] = (int)lazy_sub(lazy_sub((unsigned)v[k], q2), q);
     } else {
         const unsigned cq = a.cq;
 #pragma unroll
@@ -325,13 +329,21 @@ __device__ __forceinline__ void epilogue(int (&v)[E], const KArgs& a) {
 }
 
 // The input prologue: canonical int32 lanes start in [0, 2q) (int16 inputs
-// stay raw; the first layer adds an offset instead).
+// stay raw; the first layer adds an offset instead).  Inputs that are residues
+// already are there: a warp reduces only when one of its coefficients is not,
+// so what it usually pays is one maximum a coefficient instead of the Barrett
+// step's two multiplies.  Every lane of the warp takes part.
 template <int FAM, int E>
 __device__ __forceinline__ void prologue(int (&v)[E], const KArgs& a) {
     if constexpr (FAM == F_C32F || FAM == F_C32I) {
         const unsigned q = (unsigned)a.q, q2 = (unsigned)a.c, cq = a.cq, k31 = (unsigned)a.in_off;
+        unsigned most = 0;
 #pragma unroll
-        for (int k = 0; k < E; ++k) v[k] = (int)canon_in32(v[k], q, q2, cq, k31);
+        for (int k = 0; k < E; ++k) most = max(most, (unsigned)v[k]);
+        if (__any_sync(0xffffffffu, most >= q2)) {
+#pragma unroll
+            for (int k = 0; k < E; ++k) v[k] = (int)canon_in32(v[k], q, q2, cq, k31);
+        }
     }
 }
 
@@ -941,6 +953,47 @@ __device__ __forceinline__ void permute_br(int (&v)[1 << EL], int* sp, int g) {
     }
 }
 
+// A thread's run of consecutive coefficients moves in 32-byte accesses (whole
+// sectors; 16-byte ones, 64 bytes apart from lane to lane, touch every sector
+// twice) when the buffer is aligned to them -- the ABI asks for 16 bytes -- and
+// in 16-byte ones otherwise.  Coefficients are read with plain loads, tables with
+// read-only ones (__ldg): a dependent launch (grid_dep_start) is resident before
+// the previous grid has written its outputs, so they are not read-only data for
+// as long as the kernel runs.
+__device__ __forceinline__ bool aligned32(const void* p) { return (reinterpret_cast<unsigned long long>(p) & 31) == 0; }
+__device__ __forceinline__ void ldg32(const void* p, int4& x, int4& y) {
+    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w), "=r"(y.x), "=r"(y.y), "=r"(y.z), "=r"(y.w)
+                 : "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ void stg32(void* p, int4 x, int4 y) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(x.x), "r"(x.y), "r"(x.z), "r"(x.w),
+                 "r"(y.x), "r"(y.y), "r"(y.z), "r"(y.w)
+                 : "memory");
+}
+// a thread's run of W 16-byte words
+template <int W>
+__device__ __forceinline__ void load_run(int4 (&w)[W], const int4* src, bool wide) {
+    if (W % 2 == 0 && wide) {
+#pragma unroll
+        for (int j = 0; j + 1 < W; j += 2) ldg32(src + j, w[j], w[j + 1]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < W; ++j) w[j] = src[j];
+    }
+}
+template <int W>
+__device__ __forceinline__ void store_run(int4* dst, const int4 (&w)[W], bool wide) {
+    if (W % 2 == 0 && wide) {
+#pragma unroll
+        for (int j = 0; j + 1 < W; j += 2) stg32(dst + j, w[j], w[j + 1]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < W; ++j) dst[j] = w[j];
+    }
+}
+
 template <bool I32, int L, int EL, int LO>
 __device__ __forceinline__ void load_poly(int (&v)[1 << EL], const KArgs& a, long long poly, int g) {
     constexpr int E = 1 << EL;
@@ -948,25 +1001,27 @@ __device__ __forceinline__ void load_poly(int (&v)[1 << EL], const KArgs& a, lon
     if constexpr (I32) {
         const int* src = static_cast<const int*>(a.in) + poly * N;
         if constexpr (LO == 0 && E >= 4) {
-            const int4* s4 = reinterpret_cast<const int4*>(src + (long long)g * E);
+            int4 ws[E / 4];
+            load_run(ws, reinterpret_cast<const int4*>(src + (long long)g * E), aligned32(a.in));
 #pragma unroll
             for (int j = 0; j < E / 4; ++j) {
-                const int4 w = __ldg(s4 + j);
+                const int4 w = ws[j];
                 v[4 * j] = w.x; v[4 * j + 1] = w.y; v[4 * j + 2] = w.z; v[4 * j + 3] = w.w;
             }
         } else {
 #pragma unroll
             for (int k = 0; k < E; ++k) {
-                v[k] = __ldg(src + posmap<LO, EL>(g, k));
+                v[k] = src[posmap<LO, EL>(g, k)];
             }
         }
     } else {
         const short* src = static_cast<const short*>(a.in) + poly * N;
         if constexpr (LO == 0 && E >= 8) {
-            const int4* s4 = reinterpret_cast<const int4*>(src + (long long)g * E);
+            int4 ws[E / 8];
+            load_run(ws, reinterpret_cast<const int4*>(src + (long long)g * E), aligned32(a.in));
 #pragma unroll
             for (int j = 0; j < E / 8; ++j) {
-                const int4 w = __ldg(s4 + j);
+                const int4 w = ws[j];
                 const int ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
@@ -977,7 +1032,7 @@ __device__ __forceinline__ void load_poly(int (&v)[1 << EL], const KArgs& a, lon
         } else {
 #pragma unroll
             for (int k = 0; k < E; ++k) {
-                v[k] = (int)__ldg(src + posmap<LO, EL>(g, k));
+                v[k] = (int)src[posmap<LO, EL>(g, k)];
             }
         }
     }
@@ -990,9 +1045,10 @@ __device__ __forceinline__ void store_poly(int (&v)[1 << EL], const KArgs& a, lo
     if constexpr (I32) {
         int* dst = static_cast<int*>(a.out) + poly * N;
         if constexpr (LO == 0 && E >= 4) {
-            int4* d4 = reinterpret_cast<int4*>(dst + (long long)g * E);
+            int4 ws[E / 4];
 #pragma unroll
-            for (int j = 0; j < E / 4; ++j) d4[j] = make_int4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            for (int j = 0; j < E / 4; ++j) ws[j] = make_int4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            store_run(reinterpret_cast<int4*>(dst + (long long)g * E), ws, aligned32(a.out));
         } else {
 #pragma unroll
             for (int k = 0; k < E; ++k) {
@@ -1002,15 +1058,16 @@ __device__ __forceinline__ void store_poly(int (&v)[1 << EL], const KArgs& a, lo
     } else {
         short* dst = static_cast<short*>(a.out) + poly * N;
         if constexpr (LO == 0 && E >= 8) {
-            int4* d4 = reinterpret_cast<int4*>(dst + (long long)g * E);
+            int4 ws[E / 8];
 #pragma unroll
             for (int j = 0; j < E / 8; ++j) {
                 int ww[4];
 #pragma unroll
                 for (int h = 0; h < 4; ++h)
                     ww[h] = (v[8 * j + 2 * h] & 0xFFFF) | (v[8 * j + 2 * h + 1] << 16);
-                d4[j] = make_int4(ww[0], ww[1], ww[2], ww[3]);
+                ws[j] = make_int4(ww[0], ww[1], ww[2], ww[3]);
             }
+            store_run(reinterpret_cast<int4*>(dst + (long long)g * E), ws, aligned32(a.out));
         } else {
 #pragma unroll
             for (int k = 0; k < E; ++k) {
@@ -1126,9 +1183,9 @@ __host__ __device__ constexpr int choose_polys(int fam, int L) {
 __host__ __device__ constexpr int kntt_min_blocks(int fam, int threads, int el) {
     if (el >= 5) return threads <= 128 ? 7 : threads <= 256 ? 4 : threads <= 512 ? 2 : 1;
     if (threads <= 128) return 10;
-    // n = 4096: 40 registers for the radix-4, canonical int16 and canonical
-    // int32 inverse code (1.69 for 1.62, 2.01 for 1.98, 3.69 for 3.58)
-    if (threads <= 256) return fam == F_R4F16 || fam == F_C16F || fam == F_C16I || fam == F_C32I ? 6 : 5;
+    // n = 4096: 40 registers for the radix-4 and canonical code (radix-4 1.69
+    // for 1.62, canonical int32 forward 3.91 for 3.82, inverse 4.09 for 4.03)
+    if (threads <= 256) return fam == F_R4F16 || fam_canon(fam) ? 6 : 5;
     return 2;
 }
 

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(P << (L2 - EL)) k_crows(const __grid_constant_
         if (active) {
             const int* src = static_cast<const int*>(a.in) + row * N2;
 #pragma unroll
-            for (int k = 0; k < E; ++k) v[k] = __ldg(src + posmap<LO0, EL>(g, k));
+            for (int k = 0; k < E; ++k) v[k] = src[posmap<LO0, EL>(g, k)];
             const int2 A = __ldg(&a.twist[r * G + g]);
             const int2* B = a.twist + (long long)n1 * G + r * E;
 #pragma unroll
@@ -150,12 +150,7 @@ __global__ void __launch_bounds__(P << (L2 - EL)) k_crows(const __grid_constant_
     } else {
         // contiguous run: thread g holds columns g E .. g E + E - 1
         if (active) {
-            const int4* src = reinterpret_cast<const int4*>(static_cast<const int*>(a.in) + row * N2) + g * (E / 4);
-#pragma unroll
-            for (int j = 0; j < E / 4; ++j) {
-                const int4 w = __ldg(src + j);
-                v[4 * j] = w.x; v[4 * j + 1] = w.y; v[4 * j + 2] = w.z; v[4 * j + 3] = w.w;
-            }
+            load_poly<true, L2, EL, 0>(v, a, row, g);
         } else {
 #pragma unroll
             for (int k = 0; k < E; ++k) v[k] = 0;
@@ -167,9 +162,7 @@ __global__ void __launch_bounds__(P << (L2 - EL)) k_crows(const __grid_constant_
     if (!active) return;                                       // no exchange follows
     if constexpr (FWD) {
         epilogue<FAM, false>(v, a);                            // the forward's last pass
-        int4* dst = reinterpret_cast<int4*>(static_cast<int*>(a.out) + row * N2) + g * (E / 4);
-#pragma unroll
-        for (int j = 0; j < E / 4; ++j) dst[j] = make_int4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        store_poly<true, L2, EL, 0>(v, a, row, g);
     } else {
         const int2 A = __ldg(&a.twist[r * G + g]);
         const int2* B = a.twist + (long long)n1 * G + r * E;
