@@ -18,12 +18,20 @@ namespace {
 // 16 coefficients per thread (measured against 32 on GB300, same box: n = 2^20
 // forward 0.77 vs 0.86 ms, inverse 0.67 vs 0.85 ms for 64 polynomials)
 constexpr int LARGE_EL = 4;
-constexpr int COLS_PER_CTA = 16;   // fewer when 16 columns would need more than 1024 threads
+__host__ __device__ constexpr int large_el(int L) { return L < LARGE_EL ? L : LARGE_EL; }
+// At least 32 columns (128-byte accesses) and 256 threads per CTA.  Rows are
+// 2^12 coefficients (2^13 for n = 2^22), as long as the row pass runs well;
+// columns are the rest, so that their pass has two windows at most.
+__host__ __device__ constexpr int large_cols(int L1) {
+    const int c = 256 >> (L1 - large_el(L1));
+    return c < 32 ? 32 : c;
+}
 
 // one CTA: COLS adjacent columns of one polynomial, G threads per column
 template <int FAM, int L1, int COLS>
-__global__ void __launch_bounds__(COLS << (L1 - LARGE_EL)) k_cols(const __grid_constant__ KArgs a, int L2) {
-    constexpr int EL = LARGE_EL, G = 1 << (L1 - EL), E = 1 << EL, NS = nsteps(FAM, L1);
+__global__ void __launch_bounds__(COLS << (L1 - large_el(L1)), kntt_min_blocks(FAM, COLS << (L1 - large_el(L1)), LARGE_EL))
+    k_cols(const __grid_constant__ KArgs a, int L2) {
+    constexpr int EL = large_el(L1), G = 1 << (L1 - EL), E = 1 << EL, NS = nsteps(FAM, L1);
     constexpr int LO0 = window_lo(FAM, L1, EL, 0), LOZ = window_lo(FAM, L1, EL, NS - 1);
     extern __shared__ int csmem[];
     grid_dep_start();
@@ -36,7 +44,7 @@ __global__ void __launch_bounds__(COLS << (L1 - LARGE_EL)) k_cols(const __grid_c
     int* out = static_cast<int*>(a.out) + base;
     int v[E];
 #pragma unroll
-    for (int k = 0; k < E; ++k) v[k] = __ldg(in + ((long long)posmap<LO0, EL>(g, k) << L2));
+    for (int k = 0; k < E; ++k) v[k] = in[(long long)posmap<LO0, EL>(g, k) << L2];
     const KC kc = make_kc(a);
     run_steps_x<FAM, L1, EL, COLS, false>(v, csmem, g, kc, 0, cl, std::make_integer_sequence<int, NS>{});
     epilogue_all<false>(v, a);
@@ -47,7 +55,8 @@ __global__ void __launch_bounds__(COLS << (L1 - LARGE_EL)) k_cols(const __grid_c
 
 // one CTA: P rows of 2^L2 coefficients, G threads per row
 template <int FAM, int L2, int P>
-__global__ void __launch_bounds__(P << (L2 - LARGE_EL)) k_rows(const __grid_constant__ KArgs a, int L1) {
+__global__ void __launch_bounds__(P << (L2 - LARGE_EL), kntt_min_blocks(FAM, P << (L2 - LARGE_EL), LARGE_EL))
+    k_rows(const __grid_constant__ KArgs a, int L1) {
     constexpr int EL = LARGE_EL, G = 1 << (L2 - EL), E = 1 << EL, NS = nsteps(FAM, L2), N = 1 << L2;
     constexpr int LO0 = window_lo(FAM, L2, EL, 0), LOZ = window_lo(FAM, L2, EL, NS - 1);
     extern __shared__ int rsmem[];
@@ -58,30 +67,16 @@ __global__ void __launch_bounds__(P << (L2 - LARGE_EL)) k_rows(const __grid_cons
     const int hi = (int)(row & ((1LL << L1) - 1));               // row index inside its polynomial
     int* sp = rsmem + lp * xwords(L2);
     int v[E];
-    // rows are contiguous: every thread moves E consecutive coefficients with
-    // 16-byte accesses, and the exchange buffer turns them into (and back
-    // from) the transform's first (last) window
     if (active) {
-        const int4* src = reinterpret_cast<const int4*>(static_cast<const int*>(a.in) + row * N) + g * (E / 4);
-#pragma unroll
-        for (int j = 0; j < E / 4; ++j) {
-            const int4 w = __ldg(src + j);
-            v[4 * j] = w.x; v[4 * j + 1] = w.y; v[4 * j + 2] = w.z; v[4 * j + 3] = w.w;
-        }
+        load_poly<true, L2, EL, LO0>(v, a, row, g);
     } else {
 #pragma unroll
         for (int k = 0; k < E; ++k) v[k] = 0;
     }
-    if constexpr (LO0 != 0) exchange_windows<L2, EL, 0, LO0>(v, sp, g);
     const KC kc = make_kc(a);
     run_steps_x<FAM, L2, EL, 0, true>(v, sp, g, kc, hi, 0, std::make_integer_sequence<int, NS>{});
     epilogue_all<false>(v, a);
-    if constexpr (LOZ != 0) exchange_windows<L2, EL, LOZ, 0>(v, sp, g);
-    if (active) {
-        int4* dst = reinterpret_cast<int4*>(static_cast<int*>(a.out) + row * N) + g * (E / 4);
-#pragma unroll
-        for (int j = 0; j < E / 4; ++j) dst[j] = make_int4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-    }
+    if (active) store_poly<true, L2, EL, LOZ>(v, a, row, g);
 }
 
 template <int FAM, int L1, int L2>
@@ -89,13 +84,12 @@ LargeInfo make_large() {
     LargeInfo li;
     li.L1 = L1;
     li.L2 = L2;
-    constexpr int C = (COLS_PER_CTA << (L1 - LARGE_EL)) > 1024 ? (1024 >> (L1 - LARGE_EL)) : COLS_PER_CTA;
+    constexpr int EL1 = large_el(L1), C = large_cols(L1);
     li.cols = reinterpret_cast<const void*>(&k_cols<FAM, L1, C>);
-    li.cols_threads = C << (L1 - LARGE_EL);
-    li.cols_smem = C * (1 << L1) * 4;
+    li.cols_threads = C << (L1 - EL1);
+    li.cols_smem = num_windows(FAM, L1, EL1) > 1 ? C * (1 << L1) * 4 : 0;
     li.cols_per_cta = C;
-    constexpr int G2 = 1 << (L2 - LARGE_EL);
-    constexpr int P = G2 >= 256 ? 1 : 256 / G2;
+    constexpr int G2 = 1 << (L2 - LARGE_EL), P = 1;
     li.rows = reinterpret_cast<const void*>(&k_rows<FAM, L2, P>);
     li.rows_threads = P * G2;
     li.rows_smem = P * xwords(L2) * 4;
@@ -106,13 +100,13 @@ LargeInfo make_large() {
 template <int FAM>
 LargeInfo large_for(int L) {
     switch (L) {
-    case 16: return make_large<FAM, 8, 8>();
-    case 17: return make_large<FAM, 9, 8>();
-    case 18: return make_large<FAM, 9, 9>();
-    case 19: return make_large<FAM, 10, 9>();
-    case 20: return make_large<FAM, 10, 10>();
-    case 21: return make_large<FAM, 11, 10>();
-    case 22: return make_large<FAM, 11, 11>();
+    case 16: return make_large<FAM, 4, 12>();
+    case 17: return make_large<FAM, 5, 12>();
+    case 18: return make_large<FAM, 6, 12>();
+    case 19: return make_large<FAM, 7, 12>();
+    case 20: return make_large<FAM, 8, 12>();
+    case 21: return make_large<FAM, 9, 12>();
+    case 22: return make_large<FAM, 9, 13>();
     default: return LargeInfo();
     }
 }
