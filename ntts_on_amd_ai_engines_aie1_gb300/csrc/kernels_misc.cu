@@ -14,8 +14,8 @@ namespace {
 // int32, reduces y_k with twiddle root^(i k) and writes the eight results
 // (de-interleaved and 3-bit reversed, :152-154) as one 16-byte store at 8 i.
 // W = 2: a thread takes two adjacent i (n >= 16), so its inputs arrive as
-// 4-byte pairs, its twiddles as 16-byte pairs and its outputs leave as two
-// 16-byte stores (65536 x 4096: 2.9 TB/s with one i per thread).
+// 4-byte pairs, its twiddles as 16-byte pairs and its outputs leave as one
+// 32-byte store (65536 x 4096: 2.9 TB/s with one i per thread).
 template <int W>
 __global__ void __launch_bounds__(256) k_r8_stage(const KArgs a, int L) {
     grid_dep_start();
@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(256) k_r8_stage(const KArgs a, int L) {
     const long long total = a.batch << GL;
     const short* in = static_cast<const short*>(a.in);
     short* out = static_cast<short*>(a.out);
+    const bool wide = W == 2 && aligned32(out);
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (long long)gridDim.x * blockDim.x) {
         const long long poly = idx >> GL;
@@ -33,11 +34,11 @@ __global__ void __launch_bounds__(256) k_r8_stage(const KArgs a, int L) {
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
             if constexpr (W == 2) {
-                const int v = __ldg(reinterpret_cast<const int*>(src + m * M));
+                const int v = *reinterpret_cast<const int*>(src + m * M);
                 x[0][m] = (short)(v & 0xFFFF);
                 x[1][m] = v >> 16;
             } else {
-                x[0][m] = __ldg(src + m * M);
+                x[0][m] = src[m * M];
             }
         }
 #pragma unroll
@@ -87,15 +88,15 @@ __global__ void __launch_bounds__(256) k_r8_stage(const KArgs a, int L) {
                 o[w][brev_c<3>(k)] = z;
             }
         }
+        int4 v[W];
 #pragma unroll
         for (int w = 0; w < W; ++w) {
-            int4 v;
-            v.x = (o[w][0] & 0xFFFF) | (o[w][1] << 16);
-            v.y = (o[w][2] & 0xFFFF) | (o[w][3] << 16);
-            v.z = (o[w][4] & 0xFFFF) | (o[w][5] << 16);
-            v.w = (o[w][6] & 0xFFFF) | (o[w][7] << 16);
-            *reinterpret_cast<int4*>(out + poly * n + 8 * (i + w)) = v;
+            v[w].x = (o[w][0] & 0xFFFF) | (o[w][1] << 16);
+            v[w].y = (o[w][2] & 0xFFFF) | (o[w][3] << 16);
+            v[w].z = (o[w][4] & 0xFFFF) | (o[w][5] << 16);
+            v[w].w = (o[w][6] & 0xFFFF) | (o[w][7] << 16);
         }
+        store_run(reinterpret_cast<int4*>(out + poly * n + 8 * i), v, wide);
     }
 }
 
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(256) k_bitrev(const KArgs a, int L, int P) {
     short* dst = static_cast<short*>(a.out) + poly0 * n;
     if (n >= 8) {
         for (int j = threadIdx.x; j < count / 8; j += blockDim.x)
-            reinterpret_cast<int4*>(sb)[j] = __ldg(reinterpret_cast<const int4*>(src) + j);
+            reinterpret_cast<int4*>(sb)[j] = reinterpret_cast<const int4*>(src)[j];
     } else {
         for (int j = threadIdx.x; j < count; j += blockDim.x) sb[j] = src[j];
     }
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(BR_THREADS) k_bitrev_t(const KArgs a, int L, l
         const long long poly = t >> m;
         const int b = (int)(t & ((1 << m) - 1));
         const long long src = (poly << L) + ((long long)row << (m + K)) + ((long long)b << K) + c8;
-        const int4 w = __ldg(reinterpret_cast<const int4*>(in + src));
+        const int4 w = *reinterpret_cast<const int4*>(in + src);
         const int ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(256) k_full_barrett(const KArgs a, long long t
     const long long nvec = total >> 3;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < nvec; j += stride) {
-        const int4 w = __ldg(reinterpret_cast<const int4*>(in) + j);
+        const int4 w = reinterpret_cast<const int4*>(in)[j];
         int ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
         for (int h = 0; h < 4; ++h) {

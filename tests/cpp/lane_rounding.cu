@@ -1,7 +1,7 @@
 // Host-side check of the lane arithmetic of device.cuh against the rounding it
 // stands for, round(p / 2^K) with ties toward zero written with the product's
 // own sign: the int16 forms over every lane value and a spread of multipliers
-// (every tie of them among the values), the int32 form at constructed ties and
+// (every tie of them among the values), the int32 forms at constructed ties and
 // on a pseudo-random sample; and the bound that lets the radix-2 int16
 // butterflies of moduli below 2^14 leave out the int16 wrap.
 #include <cstdint>
@@ -45,11 +45,15 @@ int main() {
             while (!((b >> z) & 1)) ++z;
             const int32_t a = (int32_t)((uint32_t)(rnd() | 1u) << (31 - z));
             check(gbntt::rsz32(a, b) == (int32_t)round_zero((int64_t)a * b, 32), "rsz32 tie", a, b);
+            const int32_t h = (int32_t)((uint32_t)a >> 1);          // a tie of 2^31
+            check(gbntt::rsz31(h, b) == (int32_t)round_zero((int64_t)h * b, 31), "rsz31 tie", h, b);
+            check(gbntt::rsz31(-h, b) == (int32_t)round_zero((int64_t)-h * b, 31), "rsz31 tie", -h, b);
         }
     }
     for (int i = 0; i < 4000000; ++i) {
         const int32_t a = (int32_t)rnd(), b = (int32_t)rnd();
         check(gbntt::rsz32(a, b) == (int32_t)round_zero((int64_t)a * b, 32), "rsz32", a, b);
+        check(gbntt::rsz31(a, b) == (int32_t)round_zero((int64_t)a * b, 31), "rsz31", a, b);
     }
     // radix-2 butterflies of the narrow moduli: every result is an int16
     for (int q : {97, 7681, 10753, 12289, 16381}) {
