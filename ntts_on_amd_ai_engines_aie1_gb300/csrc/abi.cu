@@ -365,7 +365,7 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
         if (cl.cols) {
             n_cols = canon_table_entries(cl.L1, inverse);
             n_rows = canon_table_entries(cl.L2, inverse);
-            n_twist = canon_twist_entries(cl.L1, cl.L2, cl.row_el);
+            n_twist = canon_twist_entries(cl.L1, cl.L2, cl.row_el, cl.full_twist);
         }
         p->tab_bytes = (n_cols + n_rows + n_twist) * sizeof(int2);
         if (hp.elem_bytes == 2 && tc_supported(hp.L, hp.q)) {
@@ -391,8 +391,8 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
                 e = make_canon_table(p->d_tab + n_cols, cl.L2, q32, (uint32_t)powmod(hp.root, (uint64_t)n1, hp.q),
                                      inverse, 0);
             if (e == cudaSuccess)
-                e = make_canon_twist(p->d_tab + n_cols + n_rows, cl.L1, cl.L2, cl.row_el, q32, (uint32_t)hp.root,
-                                     inverse, 0);
+                e = make_canon_twist(p->d_tab + n_cols + n_rows, cl.L1, cl.L2, cl.row_el, cl.full_twist, q32,
+                                     (uint32_t)hp.root, inverse, 0);
             if (e == cudaSuccess) e = cudaMemsetAsync(p->d_err, 0, 256, 0);
         } else {
             e = make_canon_table(p->d_tab, hp.L, q32, (uint32_t)hp.root, inverse, 0);

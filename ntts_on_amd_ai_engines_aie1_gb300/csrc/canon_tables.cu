@@ -49,10 +49,10 @@ __global__ void k_canon_table(int2* tab, int L, unsigned q, unsigned root, int i
 // forward transform (root^-... for the inverse), split as rho^s = A[hi][s mod G]
 // * B[hi][s div G] with G = 2^(L2 - EL) (thread part) and E = 2^EL (register
 // part): A at [hi * G + t], B after all A entries at [2^L1 G + hi * E + k].
-__global__ void k_canon_twist(int2* tab, int L1, int L2, int EL, unsigned q, unsigned root, int inverse) {
+// G = 2^L2 (EL = 0) with no B part is the full table: rho^s at [hi 2^L2 + s].
+__global__ void k_canon_twist(int2* tab, int L1, int L2, int EL, int count, unsigned q, unsigned root, int inverse) {
     const int G = 1 << (L2 - EL), E = 1 << EL, R = 1 << L1;
     const unsigned long long n = 1ull << (L1 + L2);
-    const int count = R * (G + E);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         int hi;
         unsigned long long s;
@@ -85,12 +85,15 @@ cudaError_t make_canon_table(int2* d_tab, int L, uint32_t q, uint32_t root, bool
     return cudaGetLastError();
 }
 
-size_t canon_twist_entries(int L1, int L2, int EL) { return ((size_t)1 << L1) * (((size_t)1 << (L2 - EL)) + ((size_t)1 << EL)); }
+size_t canon_twist_entries(int L1, int L2, int EL, bool full) {
+    if (full) return (size_t)1 << (L1 + L2);
+    return ((size_t)1 << L1) * (((size_t)1 << (L2 - EL)) + ((size_t)1 << EL));
+}
 
-cudaError_t make_canon_twist(int2* d_tab, int L1, int L2, int EL, uint32_t q, uint32_t root, bool inverse,
+cudaError_t make_canon_twist(int2* d_tab, int L1, int L2, int EL, bool full, uint32_t q, uint32_t root, bool inverse,
                              cudaStream_t s) {
-    k_canon_twist<<<grid_of((long long)canon_twist_entries(L1, L2, EL)), 256, 0, s>>>(d_tab, L1, L2, EL, q, root,
-                                                                                     inverse ? 1 : 0);
+    const long long count = (long long)canon_twist_entries(L1, L2, EL, full);
+    k_canon_twist<<<grid_of(count), 256, 0, s>>>(d_tab, L1, L2, full ? 0 : EL, (int)count, q, root, inverse ? 1 : 0);
     return cudaGetLastError();
 }
 

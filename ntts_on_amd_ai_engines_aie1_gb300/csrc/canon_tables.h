@@ -13,8 +13,9 @@ size_t canon_table_entries(int L, bool inverse);
 cudaError_t make_canon_table(int2* d_tab, int L, uint32_t q, uint32_t root, bool inverse, cudaStream_t s);
 
 // the four-step twist of a two-pass transform of 2^(L1+L2) coefficients
-size_t canon_twist_entries(int L1, int L2, int EL);
-cudaError_t make_canon_twist(int2* d_tab, int L1, int L2, int EL, uint32_t q, uint32_t root, bool inverse,
+// (full: a pair per coefficient, row by row; else the thread and register factors)
+size_t canon_twist_entries(int L1, int L2, int EL, bool full);
+cudaError_t make_canon_twist(int2* d_tab, int L1, int L2, int EL, bool full, uint32_t q, uint32_t root, bool inverse,
                              cudaStream_t s);
 
 }  // namespace gbntt

@@ -1248,8 +1248,9 @@ struct CanonLarge {
     const void* cols = nullptr;   // k_ccols: TMA-tiled column pass
     const void* rows = nullptr;   // k_crows: row pass with the twist
     int cols_threads = 0, cols_smem = 0, cols_width = 0;   // columns per CTA
-    int rows_threads = 0, rows_smem = 0, rows_per_cta = 0;
+    int rows_threads = 0, rows_smem = 0;                   // a row per CTA
     int L1 = 0, L2 = 0, row_el = 0;
+    bool full_twist = false;      // the twist table has a pair per coefficient
 };
 CanonLarge canon_large_info(int fam, int L);
 // the four-step launches of one call: `in` -> `out` (in place allowed);

@@ -19,9 +19,15 @@
 // (cp.async.bulk.tensor.2d, an mbarrier with a bounded wait for the load, a
 // bulk-group store); with lane = column every shared-memory access of a warp
 // touches 32 distinct banks.  The row pass reads and writes whole rows with
-// coalesced accesses and applies the twist as two Shoup multiplications by
-// factors from two small tables (the twist of row r at column c = t + G k, with
-// t the thread's column and k its register, is A[r][t] * B[r][k]).
+// coalesced accesses and applies the twist.  Up to 2^20 coefficients the plan
+// holds one pair for each coefficient (8 n bytes) and the twist is one Shoup
+// multiplication; beyond, it is two, by factors from two small tables (the
+// twist of row r at column c = t + G k, with t the thread's column and k its
+// register, is A[r][t] * B[r][k]).  The passes are bound by the multiply pipe
+// (a Shoup multiplication over 2^26 coefficients measures 0.014 ms), so the
+// larger table pays as long as L2 holds it beside the chunk: rows of 2^12
+// 0.173 -> 0.160 ms forward, 0.155 -> 0.151 ms inverse; whole transforms of 2^21
+// read 0.5 % either way and of 2^22 1 % slower, so these keep the two factors.
 #include <cuda.h>
 
 #include "canon_tables.h"
@@ -108,12 +114,44 @@ __global__ void __launch_bounds__(COLS << (L1 - EL))
     }
 }
 
-// the row pass: P rows of N2 coefficients per CTA, G = N2 / 2^EL threads per
-// row; rows are numbered over the whole call, row r of its polynomial = r mod n1
-template <int FAM, int L2, int EL, int P>
-__global__ void __launch_bounds__(P << (L2 - EL)) k_crows(const __grid_constant__ KArgs a, int L1, long long row0,
-                                                          long long rows) {
-    constexpr int G = 1 << (L2 - EL), E = 1 << EL, N2 = 1 << L2, NS = nsteps(FAM, L2);
+// v[k] of row r at column g + G k times its twist (in [0, 2q)): FULL reads the
+// pair of every coefficient, otherwise the thread's and the register's factor
+template <int L2, int EL, bool FULL>
+__device__ __forceinline__ void twist_row(int* v, const KArgs& a, int n1, int r, int g) {
+    constexpr int G = 1 << (L2 - EL), E = 1 << EL;
+    const unsigned q = (unsigned)a.q;
+    if constexpr (FULL) {
+        const int2* T = a.twist + ((long long)r << L2) + g;
+#pragma unroll
+        for (int k = 0; k < E; ++k) {
+            const int2 t = __ldg(T + k * G);
+            v[k] = (int)shoup_mul((unsigned)v[k], (unsigned)t.x, (unsigned)t.y, q);
+        }
+    } else {
+        const int2 A = __ldg(&a.twist[r * G + g]);
+        const int2* B = a.twist + (long long)n1 * G + r * E;
+#pragma unroll
+        for (int k = 0; k < E; ++k) {
+            const int2 b = __ldg(B + k);
+            v[k] = (int)shoup_mul(shoup_mul((unsigned)v[k], (unsigned)A.x, (unsigned)A.y, q), (unsigned)b.x,
+                                  (unsigned)b.y, q);
+        }
+    }
+}
+
+// the row pass: one row of N2 coefficients per CTA of N2 / 2^EL threads; rows
+// are numbered over the whole call, row r of its polynomial = r mod n1
+// The bound on resident threads caps the registers: 1536 (42 registers) where
+// the row's table is full, 1280 with the two factors, 1024 for rows of 2^10,
+// where more of the loads fly at once (0.125 ms against 0.127 / 0.132 with 1536).
+constexpr int rows_min_blocks(int L2, int el, bool full) {
+    const int t = L2 <= 10 ? 1024 : (full ? 1536 : 1280), b = t >> (L2 - el);
+    return b > 16 ? 16 : b;
+}
+template <int FAM, int L2, int EL, bool FULL>
+__global__ void __launch_bounds__(1 << (L2 - EL), rows_min_blocks(L2, EL, FULL))
+    k_crows(const __grid_constant__ KArgs a, int L1, long long row0) {
+    constexpr int E = 1 << EL, N2 = 1 << L2, NS = nsteps(FAM, L2);
     constexpr int LO0 = window_lo(FAM, L2, EL, 0), LOZ = window_lo(FAM, L2, EL, NS - 1);
     constexpr bool FWD = topdown(FAM);
     // the twist sits on the window whose thread part is the low column bits
@@ -121,69 +159,52 @@ __global__ void __launch_bounds__(P << (L2 - EL)) k_crows(const __grid_constant_
     static_assert((FWD ? LOZ : LO0) == 0, "contiguous runs on the other side");
     extern __shared__ int rsm[];
     grid_dep_start();
-    const int tid = threadIdx.x, lp = tid / G, g = tid % G;
-    const long long row = row0 + (long long)blockIdx.x * P + lp;
-    const bool active = row < row0 + rows;
-    const int n1 = 1 << L1;
-    const int r = (int)(row & (n1 - 1));
-    int* sp = rsm + lp * xwords(L2);
-    const unsigned q = (unsigned)a.q;
+    const int g = threadIdx.x;
+    const long long row = row0 + blockIdx.x;
+    const int n1 = 1 << L1, r = (int)(row & (n1 - 1));
     int v[E];
     if constexpr (FWD) {
         // strided window: thread g holds columns g + G k
-        if (active) {
-            const int* src = static_cast<const int*>(a.in) + row * N2;
+        const int* src = static_cast<const int*>(a.in) + row * N2;
 #pragma unroll
-            for (int k = 0; k < E; ++k) v[k] = src[posmap<LO0, EL>(g, k)];
-            const int2 A = __ldg(&a.twist[r * G + g]);
-            const int2* B = a.twist + (long long)n1 * G + r * E;
-#pragma unroll
-            for (int k = 0; k < E; ++k) {
-                const int2 b = __ldg(B + k);
-                v[k] = (int)shoup_mul(shoup_mul((unsigned)v[k], (unsigned)A.x, (unsigned)A.y, q), (unsigned)b.x,
-                                      (unsigned)b.y, q);
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < E; ++k) v[k] = 0;
-        }
+        for (int k = 0; k < E; ++k) v[k] = src[posmap<LO0, EL>(g, k)];
+        twist_row<L2, EL, FULL>(v, a, n1, r, g);
     } else {
-        // contiguous run: thread g holds columns g E .. g E + E - 1
-        if (active) {
-            load_poly<true, L2, EL, 0>(v, a, row, g);
-        } else {
-#pragma unroll
-            for (int k = 0; k < E; ++k) v[k] = 0;
-        }
+        load_poly<true, L2, EL, 0>(v, a, row, g);              // thread g: columns g E .. g E + E - 1
         prologue<FAM>(v, a);                                   // raw input (the first pass)
     }
     const KC kc = make_kc(a);
-    run_steps<FAM, L2, EL>(v, sp, g, kc, 0, true, std::make_integer_sequence<int, NS>{});   // sp untouched so far
-    if (!active) return;                                       // no exchange follows
+    run_steps<FAM, L2, EL>(v, rsm, g, kc, 0, true, std::make_integer_sequence<int, NS>{});   // rsm untouched so far
     if constexpr (FWD) {
         epilogue<FAM, false>(v, a);                            // the forward's last pass
         store_poly<true, L2, EL, 0>(v, a, row, g);
     } else {
-        const int2 A = __ldg(&a.twist[r * G + g]);
-        const int2* B = a.twist + (long long)n1 * G + r * E;
+        twist_row<L2, EL, FULL>(v, a, n1, r, g);
         int* dst = static_cast<int*>(a.out) + row * N2;
 #pragma unroll
-        for (int k = 0; k < E; ++k) {
-            const int2 b = __ldg(B + k);
-            dst[posmap<LOZ, EL>(g, k)] = (int)shoup_mul(
-                shoup_mul((unsigned)v[k], (unsigned)A.x, (unsigned)A.y, q), (unsigned)b.x, (unsigned)b.y, q);
-        }
+        for (int k = 0; k < E; ++k) dst[posmap<LOZ, EL>(g, k)] = v[k];
     }
 }
 
-// split of 2^L: rows of 2^12 (2^13 for L = 22), columns of the rest
-constexpr int split_l2(int L) { return L >= 22 ? 13 : 12; }
-constexpr int col_el(int L1) { return L1 <= 4 ? L1 : (L1 <= 8 ? 4 : 5); }
+// The split of 2^L.  Short rows spread their exchange barriers over more CTAs
+// of an SM (24 of 64 threads at 2^10, 6 of 256 at 2^12) as long as the columns
+// stay within two windows (2^8).  Rows alone over 2^26 coefficients: 2^9 0.139
+// ms, 2^10 0.125, 2^11 0.137, 2^12 0.160, 2^13 0.211.  Whole transforms, forward
+// / inverse, with rows of 2^12 (2^13 for 2^22), wider column tiles and two
+// twist factors before:
+//   2^16 0.263/0.240 -> 0.220/0.215 ms    2^18 0.270/0.251 -> 0.231/0.229
+//   2^20 0.292/0.274 -> 0.271/0.260       2^22 0.356/0.353 -> 0.330/0.317
+constexpr int split_l2(int L) { return L <= 18 ? 10 : (L == 19 ? 11 : 12); }
+constexpr int col_el(int L1) { return L1 <= 7 ? (L1 < 4 ? L1 : 4) : 5; }
+// Columns per CTA: two warps, at least 16 columns (64 bytes of a row), tiles of
+// at most 32 KB.  Over 2^26 coefficients: 2^8 x 32 0.115 ms (16 coefficients per
+// thread), x 16 0.102, x 8 0.116; 2^7 x 32 0.103, x 16 0.094; 2^5 x 32 0.091,
+// x 16 0.139; 2^9 x 32 0.149, x 16 0.123; 2^10 x 16 0.160, x 8 0.148.
 constexpr int col_width(int L1) {
-    const int G = 1 << (L1 - col_el(L1));
-    const int c = 256 / G;
-    return c < 32 ? 32 : (c > 256 ? 256 : c);
+    const int G = 1 << (L1 - col_el(L1)), w = 64 / G < 16 ? 16 : 64 / G;
+    return (w << L1) > 8192 ? 8192 >> L1 : w;
 }
+constexpr bool full_twist(int L) { return L <= 20; }
 
 template <int FAM, int L>
 CanonLarge make_canon_large() {
@@ -197,10 +218,10 @@ CanonLarge make_canon_large() {
     li.cols_threads = COLS << (L1 - ELC);
     li.cols_smem = (1 << L1) * COLS * 4 + 16;
     li.cols_width = COLS;
-    li.rows = reinterpret_cast<const void*>(&k_crows<FAM, L2, ROW_EL, 1>);
+    li.rows = reinterpret_cast<const void*>(&k_crows<FAM, L2, ROW_EL, full_twist(L)>);
     li.rows_threads = 1 << (L2 - ROW_EL);
     li.rows_smem = xwords(L2) * 4;
-    li.rows_per_cta = 1;
+    li.full_twist = full_twist(L);
     return li;
 }
 
@@ -300,9 +321,8 @@ cudaError_t launch_canon_large(const CanonLarge& li, const KArgs& base, const in
         auto rowsk = [&](const void* src) {
             ar.in = src;
             ar.out = out;
-            void* args[] = {&ar, &L1, const_cast<long long*>(&row0), const_cast<long long*>(&rows)};
-            return launch(li.rows, (unsigned)((rows + li.rows_per_cta - 1) / li.rows_per_cta), li.rows_threads,
-                          li.rows_smem, args);
+            void* args[] = {&ar, &L1, const_cast<long long*>(&row0)};
+            return launch(li.rows, (unsigned)rows, li.rows_threads, li.rows_smem, args);
         };
         if (!inverse) {
             e = cols();
