@@ -29,14 +29,17 @@ struct gbntt_plan {
     bool br = false;       // bit-reversed load and store (radix-4 inverse)
     KernelInfo ki;
     KernelInfo kl;         // latency form for launches of at most one CTA per SM (fn nullptr: none)
-    LargeInfo large;       // int32 n >= 2^16: two-pass schedule (large.cols != nullptr)
-    CanonLarge clarge;     // canonical int32 n >= 2^16: four-step (clarge.cols != nullptr)
+    LargeInfo large;       // int32 n >= 2^14: two-pass schedule (large.cols != nullptr)
+    CanonLarge clarge;     // canonical int32 n >= 2^14: four-step (clarge.cols != nullptr)
+    uint64_t two_pass_max = 0;        // calls of more polynomials than this run one CTA per polynomial
+    const int2* tab_cols = nullptr;   // four-step: the column transforms' table (inside d_tab)
     const int2* tab_rows = nullptr;   // four-step: the row transforms' table (inside d_tab)
     const int2* twist = nullptr;      // four-step: twist factors (inside d_tab)
     unsigned* d_err = nullptr;        // four-step: set when a bounded wait ran out
     KArgs base;            // constants shared by every launch
     int2* d_tab = nullptr;
     size_t tab_bytes = 0;
+    size_t tile_tab_bytes = 0;   // of these, the table of the one-CTA kernels (first in d_tab)
     size_t tc_bytes = 0;   // tensor-core table behind it in the same allocation
     const void* tc_fn = nullptr;   // tensor-core kernel (canonical int16, n = 2^5 .. 2^10)
     int device = 0;
@@ -87,16 +90,38 @@ KernelInfo kernel_for(int fam, int L, bool br, bool lat) {
     }
 }
 
-// Canonical int32 lengths from 2^L on run as the four-step (two passes);
-// shorter ones (up to 2^15) in one CTA per polynomial.  GBNTT_FOURSTEP_MIN_L
-// (14 .. 16) overrides the default, read once per process.
-int fourstep_min_L() {
-    static const int v = [] {
-        const char* e = std::getenv("GBNTT_FOURSTEP_MIN_L");
-        const int x = e ? std::atoi(e) : 16;
-        return x >= 14 && x <= 16 ? x : 16;
+int sm_count() {
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n > 0 ? n : 1;
     }();
-    return v;
+    return sms;
+}
+
+// The largest call, in polynomials, that an int32 plan of 2^L coefficients
+// runs in two passes (0: none, UINT64_MAX: every one); 2^14 and 2^15 also fit
+// one CTA per polynomial, 2^16 and more do not.  One CTA takes the same time
+// for 1 polynomial as for 152 and keeps half an SM's threads waiting at its
+// barriers; two passes spread a polynomial over 16 .. 64 CTAs.  Measured (us,
+// one CTA -> two passes; 1 / 76 / 152 / 2^26 n^-1 polynomials):
+//   canonical 2^14  15.0 / 15.0 / 17.0 / 193 -> 10.9 / 14.0 / 17.0 / 215
+//   canonical 2^15  21.1 / 23.2 / 25.2 / 240 -> 10.9 / 18.0 / 25.2 / 224
+//   lanes 2^14      18.0 / 19.0 / 19.1 / 302 -> 10.9 / 16.0 / 21.1 / 324
+//   lanes 2^15      33.4 / 33.4 / 35.5 / 388 -> 10.9 / 22.1 / 33.4 / 343
+// so 2^15 always takes two passes and 2^14 up to half a polynomial per SM.  GBNTT_FOURSTEP_MIN_L (14 .. 16, read once per process) instead runs
+// canonical lengths from 2^that on in two passes and shorter ones in one CTA.
+uint64_t two_pass_limit(int L, bool canon) {
+    static const int env = [] {
+        const char* e = std::getenv("GBNTT_FOURSTEP_MIN_L");
+        const int x = e ? std::atoi(e) : 0;
+        return x >= 14 && x <= 16 ? x : 0;
+    }();
+    if (L < 14) return 0;
+    if (L >= 16) return UINT64_MAX;
+    if (canon && env) return L >= env ? UINT64_MAX : 0;
+    return L == 15 ? UINT64_MAX : (uint64_t)(sm_count() / 2);
 }
 
 int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, cudaStream_t s) {
@@ -105,15 +130,15 @@ int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, c
     a.out = d_out;
     a.batch = (long long)batch;
     cudaError_t e = cudaSuccess;
-    if (p->clarge.cols) {
+    if (p->clarge.cols && batch <= p->two_pass_max) {
         const bool inverse = (p->hp.kind == K_R2_I32_INV);
         int nl = 0;
-        e = launch_canon_large(p->clarge, a, p->d_tab, p->tab_rows, p->twist, d_in, d_out, (long long)batch, inverse,
+        e = launch_canon_large(p->clarge, a, p->tab_cols, p->tab_rows, p->twist, d_in, d_out, (long long)batch, inverse,
                                p->d_err, s, &nl);
         if (e != cudaSuccess) return cuda_fail(e, "four-step launch");
         g_launches.fetch_add((unsigned long long)nl, std::memory_order_relaxed);
         return GBNTT_OK;
-    } else if (p->large.cols) {
+    } else if (p->large.cols && batch <= p->two_pass_max) {
         // two passes per chunk of polynomials; a chunk (large_chunk_bytes())
         // stays in L2 between its passes.  Forward: columns then rows; inverse:
         // rows first.  Programmatic dependent launches (grid_dep_start).
@@ -163,12 +188,7 @@ int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, c
         // the design has one, and its CTAs pull the table into L1 up front (a
         // large launch finds it there already, and the extra prefetches
         // measured 6-8 % slower for int32 and radix-8).
-        static const int sms = [] {
-            int dev = 0, n = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-            return n > 0 ? n : 1;
-        }();
+        const int sms = sm_count();
         const bool small = batch <= (uint64_t)sms;
         if (p->tc_fn) {
             const unsigned long long tiles = ((batch << p->hp.L) + TC_TILE - 1) / TC_TILE;
@@ -187,7 +207,7 @@ int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, c
         const KernelInfo& k = small && p->kl.fn ? p->kl : p->ki;
         const unsigned long long blocks = (batch + k.polys - 1) / k.polys;
         if (blocks > 0x7FFFFFFFull) return fail(GBNTT_ERR_ARG, "batch too large for one launch");
-        a.tab_bytes = blocks <= (unsigned long long)sms ? (int)p->tab_bytes : 0;
+        a.tab_bytes = blocks <= (unsigned long long)sms ? (int)p->tile_tab_bytes : 0;
         void* args[] = {&a};
         e = launch_kernel(k.fn, (unsigned)blocks, k.threads, k.smem, args, s, true);
     } else if (p->hp.kind == K_R8_I16_STAGE) {
@@ -292,26 +312,22 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
     const bool canon = canonical_fast(kind, hp.q, flags);
     p->fam = canon ? canonical_family(kind) : family_of(kind);
     p->br = !canon && (kind == K_R4_I16_INV);
-    if (canon && hp.elem_bytes == 4 && hp.L >= fourstep_min_L() &&
-        (hp.L >= 16 || !(flags & FLAG_NATURAL_ORDER))) {   // the four-step has no natural-order form
-        p->clarge = canon_large_info(p->fam, hp.L);
-        if (!p->clarge.cols) {
-            delete p;
-            return fail(GBNTT_ERR_LENGTH, "no kernel for this length");
-        }
-    } else if (p->fam >= 0 && hp.L >= 16) {
-        p->large = large_info(p->fam, hp.L);
-        if (!p->large.cols) {
-            delete p;
-            return fail(GBNTT_ERR_LENGTH, "no kernel for this length");
-        }
-    } else if (p->fam >= 0) {
+    if (p->fam >= 0 && hp.elem_bytes == 4 && !(flags & FLAG_NATURAL_ORDER))   // two passes have no natural-order form
+        p->two_pass_max = two_pass_limit(hp.L, canon);
+    bool found = true;
+    if (p->two_pass_max) {
+        if (canon) p->clarge = canon_large_info(p->fam, hp.L);
+        else p->large = large_info(p->fam, hp.L);
+        found = canon ? p->clarge.cols != nullptr : p->large.cols != nullptr;
+    }
+    if (p->fam >= 0 && p->two_pass_max != UINT64_MAX) {
         p->ki = kernel_for(p->fam, hp.L, p->br, false);
         p->kl = kernel_for(p->fam, hp.L, p->br, true);
-        if (!p->ki.fn) {
-            delete p;
-            return fail(GBNTT_ERR_LENGTH, "no kernel for this length");
-        }
+        found = found && p->ki.fn;
+    }
+    if (!found) {
+        delete p;
+        return fail(GBNTT_ERR_LENGTH, "no kernel for this length");
     }
     cudaError_t e = cudaGetDevice(&p->device);
     if (e != cudaSuccess) {
@@ -358,16 +374,20 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
     std::vector<uint32_t> tc_tab;
     uint32_t tc_ke = 0, tc_corr = 0;
     if (canon) {
-        // canonical families: (w, w') pairs computed on the device; the
-        // four-step holds the column and row transforms' tables and the twist
+        // canonical families: (w, w') pairs computed on the device: the table
+        // of the whole transform where one CTA may run it (batches do, at
+        // every length that fits), then for the four-step those of the column
+        // and row transforms and the twist
         const CanonLarge& cl = p->clarge;
-        size_t n_cols = canon_table_entries(hp.L, inverse), n_rows = 0, n_twist = 0;
+        const size_t n_tile = hp.L <= 15 ? canon_table_entries(hp.L, inverse) : 0;
+        size_t n_cols = 0, n_rows = 0, n_twist = 0;
         if (cl.cols) {
             n_cols = canon_table_entries(cl.L1, inverse);
             n_rows = canon_table_entries(cl.L2, inverse);
             n_twist = canon_twist_entries(cl.L1, cl.L2, cl.row_el, cl.full_twist);
         }
-        p->tab_bytes = (n_cols + n_rows + n_twist) * sizeof(int2);
+        p->tile_tab_bytes = n_tile * sizeof(int2);
+        p->tab_bytes = (n_tile + n_cols + n_rows + n_twist) * sizeof(int2);
         if (hp.elem_bytes == 2 && tc_supported(hp.L, hp.q)) {
             tc_build(hp.L, hp.q, hp.root, inverse, (flags & FLAG_NATURAL_ORDER) != 0, (flags & FLAG_SCALE_NINV) != 0,
                      tc_tab, &tc_ke, &tc_corr);
@@ -382,20 +402,20 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
                                                   : cuda_fail(e, "cudaMalloc");
         }
         const uint32_t q32 = (uint32_t)hp.q;
+        if (n_tile) e = make_canon_table(p->d_tab, hp.L, q32, (uint32_t)hp.root, inverse, 0);
         if (cl.cols) {
             const int64_t n1 = (int64_t)1 << cl.L1, n2 = (int64_t)1 << cl.L2;
-            p->tab_rows = p->d_tab + n_cols;
-            p->twist = p->d_tab + n_cols + n_rows;
-            e = make_canon_table(p->d_tab, cl.L1, q32, (uint32_t)powmod(hp.root, (uint64_t)n2, hp.q), inverse, 0);
+            int2 *tc = p->d_tab + n_tile, *tr = tc + n_cols, *tt = tr + n_rows;
+            p->tab_cols = tc;
+            p->tab_rows = tr;
+            p->twist = tt;
             if (e == cudaSuccess)
-                e = make_canon_table(p->d_tab + n_cols, cl.L2, q32, (uint32_t)powmod(hp.root, (uint64_t)n1, hp.q),
-                                     inverse, 0);
+                e = make_canon_table(tc, cl.L1, q32, (uint32_t)powmod(hp.root, (uint64_t)n2, hp.q), inverse, 0);
             if (e == cudaSuccess)
-                e = make_canon_twist(p->d_tab + n_cols + n_rows, cl.L1, cl.L2, cl.row_el, cl.full_twist, q32,
-                                     (uint32_t)hp.root, inverse, 0);
+                e = make_canon_table(tr, cl.L2, q32, (uint32_t)powmod(hp.root, (uint64_t)n1, hp.q), inverse, 0);
+            if (e == cudaSuccess)
+                e = make_canon_twist(tt, cl.L1, cl.L2, cl.row_el, cl.full_twist, q32, (uint32_t)hp.root, inverse, 0);
             if (e == cudaSuccess) e = cudaMemsetAsync(p->d_err, 0, 256, 0);
-        } else {
-            e = make_canon_table(p->d_tab, hp.L, q32, (uint32_t)hp.root, inverse, 0);
         }
         if (e == cudaSuccess && p->tc_bytes)
             e = cudaMemcpyAsync(reinterpret_cast<char*>(p->d_tab) + p->tab_bytes, tc_tab.data(), p->tc_bytes,
@@ -415,7 +435,7 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
         dev_tab = hp.tab;
     }
     if (!dev_tab.empty()) {
-        p->tab_bytes = dev_tab.size() * sizeof(int32_t);
+        p->tab_bytes = p->tile_tab_bytes = dev_tab.size() * sizeof(int32_t);
         e = cudaMalloc(&p->d_tab, p->tab_bytes);
         if (e != cudaSuccess) {
             delete p;

@@ -21,7 +21,10 @@ constexpr int LARGE_EL = 4;
 __host__ __device__ constexpr int large_el(int L) { return L < LARGE_EL ? L : LARGE_EL; }
 // At least 32 columns (128-byte accesses) and 256 threads per CTA.  Rows are
 // 2^12 coefficients (2^13 for n = 2^22), as long as the row pass runs well;
-// columns are the rest, so that their pass has two windows at most.
+// columns are the rest, so that their pass has two windows at most.  2^14, 2^17
+// and 2^18 measured faster with shorter rows (over 2^26 coefficients, forward /
+// inverse: 2^17 5+12 391/406 us, 7+10 390/386; 2^18 6+12 410/421, 7+11 408/409;
+// 64 polynomials of 2^14, 4+10 16/13 us, 5+9 14/13).
 __host__ __device__ constexpr int large_cols(int L1) {
     const int c = 256 >> (L1 - large_el(L1));
     return c < 32 ? 32 : c;
@@ -100,9 +103,11 @@ LargeInfo make_large() {
 template <int FAM>
 LargeInfo large_for(int L) {
     switch (L) {
+    case 14: return make_large<FAM, 5, 9>();
+    case 15: return make_large<FAM, 4, 11>();
     case 16: return make_large<FAM, 4, 12>();
-    case 17: return make_large<FAM, 5, 12>();
-    case 18: return make_large<FAM, 6, 12>();
+    case 17: return make_large<FAM, 7, 10>();
+    case 18: return make_large<FAM, 7, 11>();
     case 19: return make_large<FAM, 7, 12>();
     case 20: return make_large<FAM, 8, 12>();
     case 21: return make_large<FAM, 9, 12>();
