@@ -166,10 +166,10 @@ int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, c
             const unsigned cgrid = (unsigned)(np * ((1LL << li.L2) / li.cols_per_cta));
             const unsigned rgrid = (unsigned)(((np << li.L1) + li.rows_per_cta - 1) / li.rows_per_cta);
             auto cols = [&](void** args) {
-                return launch_kernel(li.cols, cgrid, li.cols_threads, li.cols_smem, args, s, true);
+                return launch_kernel(li.cols, cgrid, li.cols_threads, li.cols_smem, args, s, true, SMEM_SHARE);
             };
             auto rows = [&](void** args) {
-                return launch_kernel(li.rows, rgrid, li.rows_threads, li.rows_smem, args, s, true);
+                return launch_kernel(li.rows, rgrid, li.rows_threads, li.rows_smem, args, s, true, SMEM_SHARE);
             };
             if (!inverse) {
                 e = cols(cargs_first);

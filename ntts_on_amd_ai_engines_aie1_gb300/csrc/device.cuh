@@ -1261,9 +1261,20 @@ cudaError_t launch_canon_large(const CanonLarge& li, const KArgs& base, const in
                                unsigned* err, cudaStream_t s, int* launches);
 
 // kernels_misc.cu: fn on stream s, as a programmatic dependent launch when
-// `dependent` (see grid_dep_start)
+// `dependent` (see grid_dep_start), with the split of an SM's memory between
+// shared memory and L1 that smem_share asks for (percent; 0: the driver's choice)
 cudaError_t launch_kernel(const void* fn, unsigned grid, int threads, int smem, void** args, cudaStream_t s,
-                          bool dependent);
+                          bool dependent, int smem_share = 0);
+// An SM drains before its split between shared memory and L1 changes.  The
+// driver sizes it for each kernel by itself, so a column pass without shared
+// memory and a row pass with some, or the three unit kernels in a row, paid for
+// it between any two launches and could not overlap (grid_dep_start).  Kernels
+// that users run in alternation therefore ask for the same split: 60 %, which
+// becomes 164 KB of 228 and holds every one of them at full residency.  Driver's
+// choice -> 60 %: lane transform of 8 x 2^16 21.1 -> 13.0 us, canonical inverse of
+// 4 x 2^16 15.0 -> 11.0, of 1 x 2^20 23.2 -> 19.1; long calls within 1 %; the units
+// 173.8 -> 160.3 us over 2^26 coefficients (50 %: 163.3, 80 %: 165.5).
+constexpr int SMEM_SHARE = 60;
 // the polynomials of a call go through the two passes of the long int32
 // transforms in chunks of at most this many bytes, so the intermediate stays
 // in L2 (96 MiB; GBNTT_FOURSTEP_CHUNK_MB, 8 .. 120, read once per process)

@@ -309,10 +309,12 @@ cudaError_t launch_canon_large(const CanonLarge& li, const KArgs& base, const in
         const long long np = chunk < batch - p0 ? chunk : batch - p0;
         const long long tile0 = p0 * tpp, row0 = p0 * n1, rows = np * n1;
         int L1 = li.L1;
-        // programmatic dependent launches (grid_dep_start)
+        // programmatic dependent launches (grid_dep_start); 2^22 runs 2 % faster
+        // with the driver's own split of each pass
+        const int share = li.L1 + li.L2 < 22 ? SMEM_SHARE : 0;
         auto launch = [&](const void* fn, unsigned grid, int threads, int smem, void** args) {
             ++nl;
-            return launch_kernel(fn, grid, threads, smem, args, s, true);
+            return launch_kernel(fn, grid, threads, smem, args, s, true, share);
         };
         auto cols = [&]() {
             void* args[] = {&map_in, &map_out, &ac, const_cast<int*>(&n2), const_cast<long long*>(&tile0), &err};

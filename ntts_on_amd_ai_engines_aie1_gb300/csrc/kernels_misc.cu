@@ -238,7 +238,7 @@ cudaError_t launch_r8_stage(const KArgs& a, int L, cudaStream_t s) {
     KArgs ka = a;
     void* args[] = {&ka, &L};
     const void* fn = pair ? reinterpret_cast<const void*>(&k_r8_stage<2>) : reinterpret_cast<const void*>(&k_r8_stage<1>);
-    return launch_kernel(fn, grid_for(work, 256), 256, 0, args, s, true);
+    return launch_kernel(fn, grid_for(work, 256), 256, 0, args, s, true, SMEM_SHARE);
 }
 
 cudaError_t launch_bitrev(const KArgs& a, int L, cudaStream_t s) {
@@ -257,7 +257,7 @@ cudaError_t launch_bitrev(const KArgs& a, int L, cudaStream_t s) {
                        : K == 4 ? reinterpret_cast<const void*>(&k_bitrev_t<4>)
                        : K == 5 ? reinterpret_cast<const void*>(&k_bitrev_t<5>)
                                 : reinterpret_cast<const void*>(&k_bitrev_t<6>);
-        return launch_kernel(fn, grid, BR_THREADS, 0, args, s, true);
+        return launch_kernel(fn, grid, BR_THREADS, 0, args, s, true, SMEM_SHARE);
     }
     const int n = 1 << L;
     const int P = n >= 8192 ? 1 : 8192 / n;
@@ -273,23 +273,30 @@ cudaError_t launch_full_barrett(const KArgs& a, long long total, int fs, int wq,
     KArgs ka = a;
     void* args[] = {&ka, &total, &fs, &wq};
     return launch_kernel(reinterpret_cast<const void*>(&k_full_barrett), grid_for((total + 7) / 8, 256), 256, 0, args,
-                         s, true);
+                         s, true, SMEM_SHARE);
 }
 
 const void* bitrev_kernel_ptr() { return reinterpret_cast<const void*>(&k_bitrev); }
 
 cudaError_t launch_kernel(const void* fn, unsigned grid, int threads, int smem, void** args, cudaStream_t s,
-                          bool dependent) {
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+                          bool dependent, int smem_share) {
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (dependent) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (smem_share) {
+        attr[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[n++].val.sharedMemCarveout = (unsigned)smem_share;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = s;
-    cfg.attrs = dependent ? attr : nullptr;
-    cfg.numAttrs = dependent ? 1 : 0;
+    cfg.attrs = n ? attr : nullptr;
+    cfg.numAttrs = n;
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
