@@ -131,19 +131,19 @@ int gbntt_plan_destroy(gbntt_plan* plan);
  * per call, except the int32 designs with n >= 2^15 (up to 2^22), and with
  * n = 2^14 up to half a polynomial per SM, which run two passes (column and row
  * sub-transforms) per chunk of polynomials (at most 96 MiB, which stays in L2
- * between the passes; the canonical four-step's column pass moves 2D tiles with
- * the Tensor Memory Accelerator and its row pass applies the four-step twist).
+ * between the passes; the canonical column pass moves 2D tiles with the Tensor
+ * Memory Accelerator).
  * In natural order n = 2^14 and 2^15 run one CTA per polynomial.  The
  * environment variable GBNTT_FOURSTEP_MIN_L (14, 15 or 16, read once per
- * process) runs the canonical int32 plans of n >= 2^that length as the
- * four-step, whatever the batch, and shorter ones in one CTA per polynomial;
+ * process) runs the canonical int32 plans of n >= 2^that length in two passes,
+ * whatever the batch, and shorter ones in one CTA per polynomial;
  * GBNTT_FOURSTEP_CHUNK_MB (8 .. 120, read once) sets the chunk size of both
  * two-pass schedules. */
 int gbntt_execute(const gbntt_plan* plan, const void* d_in, void* d_out, uint64_t batch,
                   void* stream);
 
 /* Synchronous: GBNTT_ERR_TIMEOUT if a bounded wait in an earlier launch of
- * this plan ran out (the TMA tile loads of the canonical int32 four-step,
+ * this plan ran out (the TMA tile loads of the canonical int32 column pass,
  * n >= 2^14; the other designs have no waits); the call clears it. */
 int gbntt_plan_status(const gbntt_plan* plan);
 

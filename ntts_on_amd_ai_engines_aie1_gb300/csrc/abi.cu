@@ -30,12 +30,10 @@ struct gbntt_plan {
     KernelInfo ki;
     KernelInfo kl;         // latency form for launches of at most one CTA per SM (fn nullptr: none)
     LargeInfo large;       // int32 n >= 2^14: two-pass schedule (large.cols != nullptr)
-    CanonLarge clarge;     // canonical int32 n >= 2^14: four-step (clarge.cols != nullptr)
+    CanonLarge clarge;     // canonical int32 n >= 2^14: two passes (clarge.cols != nullptr)
     uint64_t two_pass_max = 0;        // calls of more polynomials than this run one CTA per polynomial
-    const int2* tab_cols = nullptr;   // four-step: the column transforms' table (inside d_tab)
-    const int2* tab_rows = nullptr;   // four-step: the row transforms' table (inside d_tab)
-    const int2* twist = nullptr;      // four-step: twist factors (inside d_tab)
-    unsigned* d_err = nullptr;        // four-step: set when a bounded wait ran out
+    const int2* tab_blocks = nullptr; // clarge: the block table (inside d_tab)
+    unsigned* d_err = nullptr;        // clarge: set when a bounded wait ran out
     KArgs base;            // constants shared by every launch
     int2* d_tab = nullptr;
     size_t tab_bytes = 0;
@@ -106,8 +104,8 @@ int sm_count() {
 // for 1 polynomial as for 152 and keeps half an SM's threads waiting at its
 // barriers; two passes spread a polynomial over 16 .. 64 CTAs.  Measured (us,
 // one CTA -> two passes; 1 / 76 / 152 / 2^26 n^-1 polynomials):
-//   canonical 2^14  15.0 / 15.0 / 17.0 / 193 -> 10.9 / 14.0 / 17.0 / 215
-//   canonical 2^15  21.1 / 23.2 / 25.2 / 240 -> 10.9 / 18.0 / 25.2 / 224
+//   canonical 2^14  15.0 / 15.0 / 17.0 / 193 -> 10.9 / 14.0 / 17.0 / 210
+//   canonical 2^15  21.1 / 23.2 / 25.2 / 240 -> 10.9 / 18.0 / 25.2 / 218
 //   lanes 2^14      18.0 / 19.0 / 19.1 / 302 -> 10.9 / 16.0 / 21.1 / 324
 //   lanes 2^15      33.4 / 33.4 / 35.5 / 388 -> 10.9 / 22.1 / 33.4 / 343
 // so 2^15 always takes two passes and 2^14 up to half a polynomial per SM.  GBNTT_FOURSTEP_MIN_L (14 .. 16, read once per process) instead runs
@@ -133,9 +131,8 @@ int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, c
     if (p->clarge.cols && batch <= p->two_pass_max) {
         const bool inverse = (p->hp.kind == K_R2_I32_INV);
         int nl = 0;
-        e = launch_canon_large(p->clarge, a, p->tab_cols, p->tab_rows, p->twist, d_in, d_out, (long long)batch, inverse,
-                               p->d_err, s, &nl);
-        if (e != cudaSuccess) return cuda_fail(e, "four-step launch");
+        e = launch_canon_large(p->clarge, a, p->tab_blocks, d_in, d_out, (long long)batch, inverse, p->d_err, s, &nl);
+        if (e != cudaSuccess) return cuda_fail(e, "two-pass launch");
         g_launches.fetch_add((unsigned long long)nl, std::memory_order_relaxed);
         return GBNTT_OK;
     } else if (p->large.cols && batch <= p->two_pass_max) {
@@ -376,25 +373,18 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
     if (canon) {
         // canonical families: (w, w') pairs computed on the device: the table
         // of the whole transform where one CTA may run it (batches do, at
-        // every length that fits), then for the four-step those of the column
-        // and row transforms and the twist
-        const CanonLarge& cl = p->clarge;
+        // every length that fits), then the block table of the two passes
         const size_t n_tile = hp.L <= 15 ? canon_table_entries(hp.L, inverse) : 0;
-        size_t n_cols = 0, n_rows = 0, n_twist = 0;
-        if (cl.cols) {
-            n_cols = canon_table_entries(cl.L1, inverse);
-            n_rows = canon_table_entries(cl.L2, inverse);
-            n_twist = canon_twist_entries(cl.L1, cl.L2, cl.row_el, cl.full_twist);
-        }
+        const size_t n_blocks = p->clarge.cols ? two_pass_entries(hp.L) : 0;
         p->tile_tab_bytes = n_tile * sizeof(int2);
-        p->tab_bytes = (n_tile + n_cols + n_rows + n_twist) * sizeof(int2);
+        p->tab_bytes = (n_tile + n_blocks) * sizeof(int2);
         if (hp.elem_bytes == 2 && tc_supported(hp.L, hp.q)) {
             tc_build(hp.L, hp.q, hp.root, inverse, (flags & FLAG_NATURAL_ORDER) != 0, (flags & FLAG_SCALE_NINV) != 0,
                      tc_tab, &tc_ke, &tc_corr);
             p->tc_bytes = tc_tab.size() * sizeof(uint32_t);
         }
         e = cudaMalloc(&p->d_tab, p->tab_bytes + p->tc_bytes);
-        if (e == cudaSuccess && cl.cols) e = cudaMalloc(&p->d_err, 256);
+        if (e == cudaSuccess && n_blocks) e = cudaMalloc(&p->d_err, 256);
         if (e != cudaSuccess) {
             if (p->d_tab) cudaFree(p->d_tab);
             delete p;
@@ -403,18 +393,11 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
         }
         const uint32_t q32 = (uint32_t)hp.q;
         if (n_tile) e = make_canon_table(p->d_tab, hp.L, q32, (uint32_t)hp.root, inverse, 0);
-        if (cl.cols) {
-            const int64_t n1 = (int64_t)1 << cl.L1, n2 = (int64_t)1 << cl.L2;
-            int2 *tc = p->d_tab + n_tile, *tr = tc + n_cols, *tt = tr + n_rows;
-            p->tab_cols = tc;
-            p->tab_rows = tr;
-            p->twist = tt;
-            if (e == cudaSuccess)
-                e = make_canon_table(tc, cl.L1, q32, (uint32_t)powmod(hp.root, (uint64_t)n2, hp.q), inverse, 0);
-            if (e == cudaSuccess)
-                e = make_canon_table(tr, cl.L2, q32, (uint32_t)powmod(hp.root, (uint64_t)n1, hp.q), inverse, 0);
-            if (e == cudaSuccess)
-                e = make_canon_twist(tt, cl.L1, cl.L2, cl.row_el, cl.full_twist, q32, (uint32_t)hp.root, inverse, 0);
+        if (n_blocks) {
+            p->tab_blocks = p->d_tab + n_tile;
+            if (e == cudaSuccess) e = 
+                e = make_two_pass_tables(p->d_tab + n_tile, hp.L, p->clarge.L2, p->clarge.row_el, q32, (uint32_t)hp.root,
+                                         inverse, 0);
             if (e == cudaSuccess) e = cudaMemsetAsync(p->d_err, 0, 256, 0);
         }
         if (e == cudaSuccess && p->tc_bytes)
@@ -517,7 +500,7 @@ int gbntt_plan_status(const gbntt_plan* p) {
     if (!w) return GBNTT_OK;
     e = cudaMemset(p->d_err, 0, sizeof(w));
     if (e != cudaSuccess) return cuda_fail(e, "status reset");
-    return fail(GBNTT_ERR_TIMEOUT, "a tile load of the four-step column pass did not arrive within the wait limit");
+    return fail(GBNTT_ERR_TIMEOUT, "a tile load of the column pass did not arrive within the wait limit");
 }
 
 int gbntt_plan_query(const gbntt_plan* p, int what, int64_t* value) {

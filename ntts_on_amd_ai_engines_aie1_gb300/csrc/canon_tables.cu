@@ -45,28 +45,25 @@ __global__ void k_canon_table(int2* tab, int L, unsigned q, unsigned root, int i
     }
 }
 
-// four-step twist factors of row hi: rho = root^(s bitrev_{L1}(hi)) for the
-// forward transform (root^-... for the inverse), split as rho^s = A[hi][s mod G]
-// * B[hi][s div G] with G = 2^(L2 - EL) (thread part) and E = 2^EL (register
-// part): A at [hi * G + t], B after all A entries at [2^L1 G + hi * E + k].
-// G = 2^L2 (EL = 0) with no B part is the full table: rho^s at [hi 2^L2 + s].
-__global__ void k_canon_twist(int2* tab, int L1, int L2, int EL, int count, unsigned q, unsigned root, int inverse) {
-    const int G = 1 << (L2 - EL), E = 1 << EL, R = 1 << L1;
-    const unsigned long long n = 1ull << (L1 + L2);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        int hi;
-        unsigned long long s;
-        if (i < R * G) {
-            hi = i / G;
-            s = (unsigned long long)(i % G);
-        } else {
-            hi = (i - R * G) / E;
-            s = (unsigned long long)((i - R * G) % E) * G;
-        }
-        const unsigned long long b = L1 ? (__brev((unsigned)hi) >> (32 - L1)) : 0;
-        unsigned long long e = (b * s) % n;
-        if (inverse && e) e = n - e;
+// 2^(L-1) entries: entry b = root^(+-bitrev(b)), L - 1 bits reversed
+__global__ void k_block_table(int2* tab, int L, unsigned q, unsigned root, int inverse) {
+    const int n = 1 << L;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n / 2; i += gridDim.x * blockDim.x) {
+        unsigned long long e = __brev((unsigned)i) >> (33 - L);
+        if (inverse && e) e = (unsigned long long)n - e;
         tab[i] = shoup_pair(powmod_dev(root, e, q), q);
+    }
+}
+
+// the tail (see canon_tables.h), from the block table
+__global__ void k_tail_table(int4* tail, const int2* tab, int L, int L2, int EL) {
+    const int g2 = L2 - EL;                                   // log2 threads of a row
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 1 << (L - 1); i += gridDim.x * blockDim.x) {
+        const int g = i & ((1 << g2) - 1), pair = (i >> g2) & ((1 << (EL - 1)) - 1), r = i >> (L2 - 1);
+        const int p = 31 - __clz(pair + 1), B = EL - 2 - p;   // 2^p pairs on bit B
+        if (B < 0) continue;                                  // the last word of each thread is unused
+        const int2* t = tab + ((((r << g2) | g) << (p + 1)) | 2 * (pair + 1 - (1 << p)));
+        tail[i] = make_int4(t[0].x, t[0].y, t[1].x, t[1].y);
     }
 }
 
@@ -85,15 +82,13 @@ cudaError_t make_canon_table(int2* d_tab, int L, uint32_t q, uint32_t root, bool
     return cudaGetLastError();
 }
 
-size_t canon_twist_entries(int L1, int L2, int EL, bool full) {
-    if (full) return (size_t)1 << (L1 + L2);
-    return ((size_t)1 << L1) * (((size_t)1 << (L2 - EL)) + ((size_t)1 << EL));
-}
+size_t two_pass_entries(int L) { return ((size_t)1 << (L - 1)) + ((size_t)1 << L); }
 
-cudaError_t make_canon_twist(int2* d_tab, int L1, int L2, int EL, bool full, uint32_t q, uint32_t root, bool inverse,
-                             cudaStream_t s) {
-    const long long count = (long long)canon_twist_entries(L1, L2, EL, full);
-    k_canon_twist<<<grid_of(count), 256, 0, s>>>(d_tab, L1, L2, full ? 0 : EL, (int)count, q, root, inverse ? 1 : 0);
+cudaError_t make_two_pass_tables(int2* d_tab, int L, int L2, int EL, uint32_t q, uint32_t root, bool inverse,
+                                 cudaStream_t s) {
+    const int grid = grid_of(1ll << (L - 1));
+    k_block_table<<<grid, 256, 0, s>>>(d_tab, L, q, root, inverse ? 1 : 0);
+    k_tail_table<<<grid, 256, 0, s>>>(reinterpret_cast<int4*>(d_tab + ((size_t)1 << (L - 1))), d_tab, L, L2, EL);
     return cudaGetLastError();
 }
 

@@ -87,16 +87,14 @@ struct KArgs {
     unsigned cq;          // floor(2^32 / q)
     int in_off;           // int16: 2M, M = q ceil(2^15 / q); int32: q - (2^31 mod q)
     unsigned ninv, ninv_q;   // n^-1 mod q and its Shoup quotient (n^-1 scaling of inverse designs)
-    union {
-        const int2* twist;    // four-step row twist factors (two-pass canonical int32 transforms)
-        const uint4* tctab;   // canonical int16: the tensor-core form's table (tc16.cuh), or nullptr
-    };
+    const uint4* tctab;   // canonical int16: the tensor-core form's table (tc16.cuh), or nullptr
 };
 
 // The scalar constants of one design, held in registers while a polynomial is
 // transformed (the matrices stay in parameter or shared memory).
 struct KC {
     const int2* tab;
+    const int4* tail;     // canonical two-pass rows: the thread's column of the tail table (canon_tables.h)
     const int* tab16;
     const int* f8;
     const int* ftail;
@@ -643,17 +641,19 @@ __device__ __forceinline__ void exchange_cols(int (&v)[1 << EL], int* sp, int g,
 // designs' blocks of the thread's run, or the canonical families' entries
 // 2^B .. 2^(B+1) - 1, when the window is the lowest bits
 template <int FAM, int FORM>
-__host__ __device__ constexpr int step_vec_pairs(int LO, int EL, int B) {
+__host__ __device__ constexpr int step_vec_pairs(int LO, int EL, int B, bool HIB) {
     if (LO != 0) return 0;
-    if (fam_canon(FAM)) return B >= 1 && B < EL ? 1 << B : 0;
-    const bool blocks = FAM == F_R2F32 || FAM == F_R2G32 || (FAM == F_R2F16 && FORM != R2_WIDE);
+    if (fam_canon(FAM) && !HIB) return B >= 1 && B < EL ? 1 << B : 0;
+    const bool blocks = fam_canon(FAM) || FAM == F_R2F32 || FAM == F_R2G32 || (FAM == F_R2F16 && FORM != R2_WIDE);
     const int n = (1 << EL) >> (B + 1);
     return blocks && n >= 2 ? n : 0;
 }
 
 // XC > 0: column pass (XC columns per CTA, exchanges through exchange_cols);
 // HIB: row pass, the polynomial is row `hi` of a longer transform and the
-// twiddle block index carries hi in its top bits.
+// twiddle block index carries hi in its top bits.  For the canonical int32
+// families HIB selects the block-indexed butterflies of the two-pass kernels,
+// in their column pass as well (hi = 0).
 // fresh: no thread of the CTA has touched sp since the CTA's last barrier, so
 // the transform's first exchange needs no leading barrier (uniform)
 template <int FAM, int L, int EL, int S, int XC = 0, bool HIB = false, int FORM = R2_WIDE>
@@ -676,14 +676,15 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
     const int q = a.q;
     // In the window on the low bits the (w, w') pairs a thread needs in one
     // layer are NV consecutive table entries: 16-byte loads take two at a time.
-    constexpr int NV = step_vec_pairs<FAM, FORM>(LO, EL, B);
+    constexpr int NV = step_vec_pairs<FAM, FORM>(LO, EL, B, HIB);
     int2 tv[NV > 0 ? NV : 1];
     if constexpr (NV > 0) {
-        const int e0 = fam_canon(FAM) ? 1 << B : ((HIB ? (hi << L) : 0) | posmap<LO, EL>(g, 0)) >> (B + 1);
+        const int e0 = fam_canon(FAM) && !HIB ? 1 << B : ((HIB ? (hi << L) : 0) | posmap<LO, EL>(g, 0)) >> (B + 1);
         const int4* src = reinterpret_cast<const int4*>(a.tab + e0);
 #pragma unroll
         for (int i = 0; i < NV / 2; ++i) {
-            const int4 w = __ldg(src + i);
+            // a row's entries of these layers lie thread by thread in the tail table
+            const int4 w = fam_canon(FAM) && HIB && XC == 0 ? __ldg(a.tail + (NV / 2 - 1 + i) * G) : __ldg(src + i);
             tv[2 * i] = make_int2(w.x, w.y);
             tv[2 * i + 1] = make_int2(w.z, w.w);
         }
@@ -691,12 +692,43 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
 #pragma unroll
     for (int r = 0; r < (E >> W); ++r) {
         const int k0 = ((r >> KB) << (KB + W)) | (r & ((1 << KB) - 1));
-        if constexpr (fam_canon(FAM)) {
+        if constexpr (fam_canon(FAM) && HIB) {
+            // Canonical butterflies of the two-pass int32 kernels.  One table
+            // serves every layer of both passes: the block of a butterfly on
+            // bit B (the position bits above it) has w = root^+-bitrev(block),
+            // so a row needs no twist between the passes.
+            static_assert(fam_i32(FAM), "the two-pass kernels are int32");
+            const int k1 = k0 | (1 << KB);
+            const unsigned uq = (unsigned)q, q2 = (unsigned)a.c;
+            const unsigned x = (unsigned)v[k0], y = (unsigned)v[k1];
+            // block 0 has w = 1; known where the registers hold the top bits
+            const bool one = XC > 0 && LO + EL == L && (k0 >> (KB + 1)) == 0;
+            int2 t = make_int2(0, 0);
+            if (!one)
+                t = NV > 0 ? tv[k0 >> (B + 1)]
+                           : __ldg(&a.tab[((hi << L) | posmap<LO, EL>(g, k0)) >> (B + 1)]);
+            if constexpr (topdown(FAM)) {
+                // Cooley-Tukey, natural order in, bit-reversed out: (x, y) ->
+                // (x + w y, x - w y).  Lanes below 4q, x brought below 2q first;
+                // the whole transform's first layer starts below 2q
+                const bool first = XC > 0 && S == 0;
+                const unsigned u = first ? x : lazy_sub(x, q2);
+                const unsigned m = first ? y : one ? lazy_sub(y, q2) : shoup_mul(y, (unsigned)t.x, (unsigned)t.y, uq);
+                v[k0] = (int)(u + m);
+                v[k1] = (int)(u + q2 - m);
+            } else {
+                // Gentleman-Sande, bit-reversed in, natural order out: (x, y) ->
+                // (x + y, (x - y) w).  Lanes below 2q, below 4q after the last layer
+                const bool last = XC > 0 && S == L - 1;
+                const unsigned s = x + y, d = x + q2 - y;
+                v[k0] = (int)(last ? s : lazy_sub(s, q2));
+                v[k1] = (int)(last ? d : one ? lazy_sub(d, q2) : shoup_mul(d, (unsigned)t.x, (unsigned)t.y, uq));
+            }
+        } else if constexpr (fam_canon(FAM)) {
             // Canonical butterflies.  Both directions index the table by the
             // position bits below the butterfly bit B, j = pos mod 2^B, at entry
             // 2^B + j, so a warp's twiddle loads are one broadcast (j from the
             // registers) or consecutive entries (j from the lane index).
-            static_assert(!HIB, "the canonical families run whole sub-transforms (the four-step twist is separate)");
             const int k1 = k0 | (1 << KB);
             // 2q comes as a value of its own: from q, every x + 2q - y
             // becomes a shift-and-add and a subtraction
@@ -914,8 +946,8 @@ __device__ __forceinline__ void run_steps(int (&v)[1 << EL], int* sp, int g, con
 
 template <int FAM, int L, int EL, int XC, bool HIB, int... S>
 __device__ __forceinline__ void run_steps_x(int (&v)[1 << EL], int* sp, int g, const KC& a, int hi, int cl,
-                                            std::integer_sequence<int, S...>) {
-    (do_step<FAM, L, EL, S, XC, HIB>(v, sp, g, a, hi, cl), ...);
+                                            std::integer_sequence<int, S...>, bool fresh = false) {
+    (do_step<FAM, L, EL, S, XC, HIB>(v, sp, g, a, hi, cl, fresh), ...);
 }
 
 // ---------------------------------------------------------------------------
@@ -1239,26 +1271,22 @@ struct LargeInfo {
 };
 LargeInfo large_info(int fam, int L);
 
-// Canonical int32 transforms of 2^14 .. 2^22 coefficients as a four-step
-// (kernels_c32_large.cu): n = n1 n2, rows of n2 coefficients.  Forward:
-// column transforms (length n1, root^n2, bit-reversed along the column), the
-// twist root^(c bitrev(r)) of row r at column c, row transforms (length n2,
-// root^n1, bit-reversed along the row).  Inverse: the same steps reversed.
+// Canonical int32 transforms of 2^14 .. 2^22 coefficients in two passes
+// (kernels_c32_large.cu): n = n1 n2, rows of n2 coefficients.  Forward: the
+// layers on the high bits as column transforms, then those on the low bits as
+// row transforms.  Inverse: the same steps reversed.
 struct CanonLarge {
     const void* cols = nullptr;   // k_ccols: TMA-tiled column pass
-    const void* rows = nullptr;   // k_crows: row pass with the twist
+    const void* rows = nullptr;   // k_crows: row pass
     int cols_threads = 0, cols_smem = 0, cols_width = 0;   // columns per CTA
     int rows_threads = 0, rows_smem = 0;                   // a row per CTA
     int L1 = 0, L2 = 0, row_el = 0;
-    bool full_twist = false;      // the twist table has a pair per coefficient
 };
 CanonLarge canon_large_info(int fam, int L);
-// the four-step launches of one call: `in` -> `out` (in place allowed);
-// tab_cols/tab_rows: the sub-transforms' tables, twist: the factors;
-// err: a device word set when a bounded wait runs out
-cudaError_t launch_canon_large(const CanonLarge& li, const KArgs& base, const int2* tab_cols, const int2* tab_rows,
-                               const int2* twist, const void* in, void* out, long long batch, bool inverse,
-                               unsigned* err, cudaStream_t s, int* launches);
+// the launches of one call: `in` -> `out` (in place allowed); tab: the block
+// table (canon_tables.h); err: a device word set when a bounded wait runs out
+cudaError_t launch_canon_large(const CanonLarge& li, const KArgs& base, const int2* tab, const void* in, void* out,
+                               long long batch, bool inverse, unsigned* err, cudaStream_t s, int* launches);
 
 // kernels_misc.cu: fn on stream s, as a programmatic dependent launch when
 // `dependent` (see grid_dep_start), with the split of an SM's memory between

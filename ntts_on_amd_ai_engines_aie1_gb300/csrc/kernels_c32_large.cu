@@ -1,16 +1,20 @@
 // kernels_c32_large.cu -- canonical int32 transforms of 2^14 .. 2^22
-// coefficients as a four-step (column pass, twist, row pass).
+// coefficients in two passes (columns, rows).
 //
-// With n = n1 n2 and the polynomial viewed as n1 rows of n2 coefficients
-// (row-major, no transpose in memory), the forward transform with output in
-// bit-reversed order is
-//   1. every column c: the length-n1 transform with root^n2, bit-reversed
-//      along the column (row r then holds frequency k1 = bitrev(r));
-//   2. the twist: row r, column c times root^(c bitrev(r));
-//   3. every row: the length-n2 transform with root^n1, bit-reversed along
-//      the row,
-// and the inverse (bit-reversed in, natural out, no n^-1) runs the inverse
-// steps in the opposite order: rows, untwist by root^-(c bitrev(r)), columns.
+// Forward: Cooley-Tukey layers on natural-order input, high position bits
+// first.  The block of a butterfly on bit B (the position bits above B) has the
+// twiddle root^bitrev(block), the bits reversed as log2(n) - 1 of them, whatever
+// the layer: the layer splits x^m - z^2 into x^(m/2) -+ z, and the root of a
+// block's left half is the next layer's entry at twice its index.  With n = n1
+// n2 and the polynomial viewed as n1 rows of n2 coefficients (row-major, no
+// transpose in memory), the layers on the high bits are transforms of the
+// columns, the same for every column, and those on the low bits are transforms
+// of the rows, whose block index carries the row in its top bits.  One table of
+// n / 2 pairs serves all of them, and nothing is multiplied between the passes;
+// a row's entries for its lowest four bits are held a second time in the order
+// in which its threads read them (the tail: 16 coalesced bytes a lane).
+// The inverse (bit-reversed in, natural out, no n^-1) undoes the layers from the
+// low bits up (Gentleman-Sande, root^-bitrev(block)): rows, then columns.
 // Polynomials go through both passes in chunks of at most large_chunk_bytes(), so the
 // intermediate stays in L2 between the passes.
 //
@@ -19,15 +23,16 @@
 // (cp.async.bulk.tensor.2d, an mbarrier with a bounded wait for the load, a
 // bulk-group store); with lane = column every shared-memory access of a warp
 // touches 32 distinct banks.  The row pass reads and writes whole rows with
-// coalesced accesses and applies the twist.  Up to 2^20 coefficients the plan
-// holds one pair for each coefficient (8 n bytes) and the twist is one Shoup
-// multiplication; beyond, it is two, by factors from two small tables (the
-// twist of row r at column c = t + G k, with t the thread's column and k its
-// register, is A[r][t] * B[r][k]).  The passes are bound by the multiply pipe
-// (a Shoup multiplication over 2^26 coefficients measures 0.014 ms), so the
-// larger table pays as long as L2 holds it beside the chunk: rows of 2^12
-// 0.173 -> 0.160 ms forward, 0.155 -> 0.151 ms inverse; whole transforms of 2^21
-// read 0.5 % either way and of 2^22 1 % slower, so these keep the two factors.
+// coalesced accesses.
+//
+// What bounds it: a butterfly's one high and two low 32-bit products hold the
+// multiply pipe for 7.6 clocks a warp, 56 % of a 2^12 row pass; its loads and
+// exchanges share the other half with the additions.  Over 2^26 coefficients,
+// forward / inverse, against the four-step that multiplies by a twist between
+// the passes (one factor per coefficient up to 2^20, two beyond):
+//   2^16 224/229 -> 224/214 us    2^18 237/239 -> 230/224
+//   2^20 275/264 -> 265/256       2^22 317/322 -> 314/313
+// Without the tail (64 contiguous bytes a lane): 2^16 236/225, 2^20 269/264.
 #include <cuda.h>
 
 #include "canon_tables.h"
@@ -99,7 +104,7 @@ __global__ void __launch_bounds__(COLS << (L1 - EL))
     for (int k = 0; k < E; ++k) v[k] = tile[posmap<LO0, EL>(g, k) * COLS + cl];
     if constexpr (FWD) prologue<FAM>(v, a);                    // raw input (the first pass)
     const KC kc = make_kc(a);
-    run_steps_x<FAM, L1, EL, COLS, false>(v, tile, g, kc, 0, cl, std::make_integer_sequence<int, NS>{});
+    run_steps_x<FAM, L1, EL, COLS, true>(v, tile, g, kc, 0, cl, std::make_integer_sequence<int, NS>{});
     if constexpr (!FWD) epilogue<FAM, false>(v, a);            // the inverse's last pass
     __syncthreads();                                           // every read of the tile is done
 #pragma unroll
@@ -114,72 +119,44 @@ __global__ void __launch_bounds__(COLS << (L1 - EL))
     }
 }
 
-// v[k] of row r at column g + G k times its twist (in [0, 2q)): FULL reads the
-// pair of every coefficient, otherwise the thread's and the register's factor
-template <int L2, int EL, bool FULL>
-__device__ __forceinline__ void twist_row(int* v, const KArgs& a, int n1, int r, int g) {
-    constexpr int G = 1 << (L2 - EL), E = 1 << EL;
-    const unsigned q = (unsigned)a.q;
-    if constexpr (FULL) {
-        const int2* T = a.twist + ((long long)r << L2) + g;
-#pragma unroll
-        for (int k = 0; k < E; ++k) {
-            const int2 t = __ldg(T + k * G);
-            v[k] = (int)shoup_mul((unsigned)v[k], (unsigned)t.x, (unsigned)t.y, q);
-        }
-    } else {
-        const int2 A = __ldg(&a.twist[r * G + g]);
-        const int2* B = a.twist + (long long)n1 * G + r * E;
-#pragma unroll
-        for (int k = 0; k < E; ++k) {
-            const int2 b = __ldg(B + k);
-            v[k] = (int)shoup_mul(shoup_mul((unsigned)v[k], (unsigned)A.x, (unsigned)A.y, q), (unsigned)b.x,
-                                  (unsigned)b.y, q);
-        }
-    }
-}
-
 // the row pass: one row of N2 coefficients per CTA of N2 / 2^EL threads; rows
-// are numbered over the whole call, row r of its polynomial = r mod n1
-// The bound on resident threads caps the registers: 1536 (42 registers) where
-// the row's table is full, 1280 with the two factors, 1024 for rows of 2^10,
-// where more of the loads fly at once (0.125 ms against 0.127 / 0.132 with 1536).
-constexpr int rows_min_blocks(int L2, int el, bool full) {
-    const int t = L2 <= 10 ? 1024 : (full ? 1536 : 1280), b = t >> (L2 - el);
+// are numbered over the whole call, row r of its polynomial = r mod n1.
+// The bound on resident threads caps the registers: 1536 (42 registers), 1024
+// for rows of 2^10, where more of the loads fly at once (0.125 ms for the pass
+// over 2^26 coefficients against 0.127 forward and 0.132 inverse with 1536).
+constexpr int rows_min_blocks(int L2, int el) {
+    const int b = (L2 <= 10 ? 1024 : 1536) >> (L2 - el);
     return b > 16 ? 16 : b;
 }
-template <int FAM, int L2, int EL, bool FULL>
-__global__ void __launch_bounds__(1 << (L2 - EL), rows_min_blocks(L2, EL, FULL))
+template <int FAM, int L2, int EL>
+__global__ void __launch_bounds__(1 << (L2 - EL), rows_min_blocks(L2, EL))
     k_crows(const __grid_constant__ KArgs a, int L1, long long row0) {
     constexpr int E = 1 << EL, N2 = 1 << L2, NS = nsteps(FAM, L2);
     constexpr int LO0 = window_lo(FAM, L2, EL, 0), LOZ = window_lo(FAM, L2, EL, NS - 1);
     constexpr bool FWD = topdown(FAM);
-    // the twist sits on the window whose thread part is the low column bits
-    static_assert((FWD ? LO0 : LOZ) == L2 - EL, "twist layout");
-    static_assert((FWD ? LOZ : LO0) == 0, "contiguous runs on the other side");
+    static_assert((FWD ? LOZ : LO0) == 0, "contiguous runs at the rows' outer side");
     extern __shared__ int rsm[];
     grid_dep_start();
     const int g = threadIdx.x;
     const long long row = row0 + blockIdx.x;
-    const int n1 = 1 << L1, r = (int)(row & (n1 - 1));
+    const int r = (int)(row & ((1 << L1) - 1));
     int v[E];
     if constexpr (FWD) {
         // strided window: thread g holds columns g + G k
         const int* src = static_cast<const int*>(a.in) + row * N2;
 #pragma unroll
         for (int k = 0; k < E; ++k) v[k] = src[posmap<LO0, EL>(g, k)];
-        twist_row<L2, EL, FULL>(v, a, n1, r, g);
     } else {
         load_poly<true, L2, EL, 0>(v, a, row, g);              // thread g: columns g E .. g E + E - 1
         prologue<FAM>(v, a);                                   // raw input (the first pass)
     }
-    const KC kc = make_kc(a);
-    run_steps<FAM, L2, EL>(v, rsm, g, kc, 0, true, std::make_integer_sequence<int, NS>{});   // rsm untouched so far
+    KC kc = make_kc(a);
+    kc.tail = reinterpret_cast<const int4*>(a.tab + (1LL << (L1 + L2 - 1))) + ((long long)r << (L2 - 1)) + g;
+    run_steps_x<FAM, L2, EL, 0, true>(v, rsm, g, kc, r, 0, std::make_integer_sequence<int, NS>{}, true);   // rsm untouched so far
     if constexpr (FWD) {
         epilogue<FAM, false>(v, a);                            // the forward's last pass
         store_poly<true, L2, EL, 0>(v, a, row, g);
     } else {
-        twist_row<L2, EL, FULL>(v, a, n1, r, g);
         int* dst = static_cast<int*>(a.out) + row * N2;
 #pragma unroll
         for (int k = 0; k < E; ++k) dst[posmap<LOZ, EL>(g, k)] = v[k];
@@ -187,13 +164,9 @@ __global__ void __launch_bounds__(1 << (L2 - EL), rows_min_blocks(L2, EL, FULL))
 }
 
 // The split of 2^L.  Short rows spread their exchange barriers over more CTAs
-// of an SM (24 of 64 threads at 2^10, 6 of 256 at 2^12) as long as the columns
-// stay within two windows (2^8).  Rows alone over 2^26 coefficients: 2^9 0.139
-// ms, 2^10 0.125, 2^11 0.137, 2^12 0.160, 2^13 0.211.  Whole transforms, forward
-// / inverse, with rows of 2^12 (2^13 for 2^22), wider column tiles and two
-// twist factors before:
-//   2^16 0.263/0.240 -> 0.220/0.215 ms    2^18 0.270/0.251 -> 0.231/0.229
-//   2^20 0.292/0.274 -> 0.271/0.260       2^22 0.356/0.353 -> 0.330/0.317
+// of an SM (16 of 64 threads at 2^10, 6 of 256 at 2^12) as long as the columns
+// stay within two windows (2^8).  Row passes alone over 2^26 coefficients,
+// with a twist: 2^9 0.139 ms, 2^10 0.125, 2^11 0.137, 2^12 0.160, 2^13 0.211.
 constexpr int split_l2(int L) { return L <= 18 ? 10 : (L == 19 ? 11 : 12); }
 constexpr int col_el(int L1) { return L1 <= 7 ? (L1 < 4 ? L1 : 4) : 5; }
 // Columns per CTA: two warps, at least 16 columns (64 bytes of a row), tiles of
@@ -204,24 +177,21 @@ constexpr int col_width(int L1) {
     const int G = 1 << (L1 - col_el(L1)), w = 64 / G < 16 ? 16 : 64 / G;
     return (w << L1) > 8192 ? 8192 >> L1 : w;
 }
-constexpr bool full_twist(int L) { return L <= 20; }
-
 template <int FAM, int L>
 CanonLarge make_canon_large() {
     constexpr int L2 = split_l2(L), L1 = L - L2;
     constexpr int ELC = col_el(L1), COLS = col_width(L1);
     CanonLarge li;
     li.L1 = L1;
-    li.L2 = L2;
     li.row_el = ROW_EL;
+    li.L2 = L2;
     li.cols = reinterpret_cast<const void*>(&k_ccols<FAM, L1, ELC, COLS>);
     li.cols_threads = COLS << (L1 - ELC);
     li.cols_smem = (1 << L1) * COLS * 4 + 16;
     li.cols_width = COLS;
-    li.rows = reinterpret_cast<const void*>(&k_crows<FAM, L2, ROW_EL, full_twist(L)>);
+    li.rows = reinterpret_cast<const void*>(&k_crows<FAM, L2, ROW_EL>);
     li.rows_threads = 1 << (L2 - ROW_EL);
     li.rows_smem = xwords(L2) * 4;
-    li.full_twist = full_twist(L);
     return li;
 }
 
@@ -281,9 +251,8 @@ CanonLarge canon_large_info(int fam, int L) {
     return CanonLarge();
 }
 
-cudaError_t launch_canon_large(const CanonLarge& li, const KArgs& base, const int2* tab_cols, const int2* tab_rows,
-                               const int2* twist, const void* in, void* out, long long batch, bool inverse,
-                               unsigned* err, cudaStream_t s, int* launches) {
+cudaError_t launch_canon_large(const CanonLarge& li, const KArgs& base, const int2* tab, const void* in, void* out,
+                               long long batch, bool inverse, unsigned* err, cudaStream_t s, int* launches) {
     const int n1 = 1 << li.L1, n2 = 1 << li.L2;
     const long long n = (long long)n1 * n2;
     const int box_rows = n1 < 256 ? n1 : 256;
@@ -301,9 +270,8 @@ cudaError_t launch_canon_large(const CanonLarge& li, const KArgs& base, const in
     if (chunk < 1) chunk = 1;
     const long long tpp = n2 / li.cols_width;
     KArgs ac = base, ar = base;
-    ac.tab = tab_cols;
-    ar.tab = tab_rows;
-    ar.twist = twist;
+    ac.tab = tab;
+    ar.tab = tab;
     int nl = 0;
     for (long long p0 = 0; p0 < batch; p0 += chunk) {
         const long long np = chunk < batch - p0 ? chunk : batch - p0;

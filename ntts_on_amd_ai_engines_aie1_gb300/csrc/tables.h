@@ -26,7 +26,7 @@ constexpr uint32_t FLAG_NATURAL_ORDER = 0x8u;
 constexpr uint32_t FLAG_SCALE_NINV = 0x10u;
 constexpr uint32_t FLAG_LANE_EXACT = 0x20u;
 
-// Largest two-pass (four-step) length of the canonical int32 family.
+// Largest two-pass length of the canonical int32 family.
 constexpr int CANON_MAX_L32 = 22;
 
 // The plan runs a canonical family (Shoup multiplication, lazy lanes, one
