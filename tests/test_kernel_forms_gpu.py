@@ -1,7 +1,7 @@
 """The forms a call can take beside the common one: two passes for 2^14 and
 2^15 coefficients, the direct batch kernels, buffers on 16- but not 32-byte
-boundaries, residues next to raw input.  Whole numbers: all comparisons are
-equalities."""
+boundaries, residues next to raw input, units over more polynomials than a grid
+holds.  Whole numbers: all comparisons are equalities."""
 import numpy as np
 import pytest
 
@@ -129,3 +129,19 @@ def test_one_raw_coefficient_among_residues(gb, orc, n, inverse):  # noqa: F811
     x = np.stack(rows).astype(np.int32)
     got = gpu_run(gb, 5 if inverse else 4, n, Q32, root, x, flags=1)
     assert np.array_equal(got.astype(np.int64), orc.ntt_exact(x, Q32, root, inverse=bool(inverse)))
+
+
+@pytest.mark.parametrize("n,count", [(16, 700001), (512, 40001), (4096, 5003)])
+def test_radix8_stage_over_many_polynomials(gb, n, count):  # noqa: F811
+    """More polynomials than the grid holds at once (a thread keeps its
+    twiddles over several of them): the first, the ones around the grid's
+    stride and the last equal their own calls."""
+    q = 12289
+    plan = gb.Plan(3, n, q, root_for(q, n))
+    g = torch.Generator(device="cuda").manual_seed(SEED + n)
+    x = torch.randint(-32768, 32768, (count, n), generator=g, device="cuda", dtype=torch.int16)
+    y = torch.full_like(x, 9)
+    plan.execute(x, y, count)
+    stride = torch.cuda.get_device_properties(0).multi_processor_count * 32 * 128 // max(1, n // 16)
+    for lo in (0, min(stride, count) - 8, count - 9):
+        assert torch.equal(y[lo:lo + 9], plan(x[lo:lo + 9].clone())), lo
