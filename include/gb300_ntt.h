@@ -130,15 +130,14 @@ int gbntt_plan_destroy(gbntt_plan* plan);
  * `stream` (a cudaStream_t; NULL = legacy default stream).  One kernel launch
  * per call, except the int32 designs with n >= 2^15 (up to 2^22), and with
  * n = 2^14 up to half a polynomial per SM, which run two passes (column and row
- * sub-transforms) per chunk of polynomials (at most 96 MiB, which stays in L2
- * between the passes; the canonical column pass moves 2D tiles with the Tensor
+ * sub-transforms; the canonical column pass moves 2D tiles with the Tensor
  * Memory Accelerator).
  * In natural order n = 2^14 and 2^15 run one CTA per polynomial.  The
  * environment variable GBNTT_FOURSTEP_MIN_L (14, 15 or 16, read once per
  * process) runs the canonical int32 plans of n >= 2^that length in two passes,
  * whatever the batch, and shorter ones in one CTA per polynomial;
- * GBNTT_FOURSTEP_CHUNK_MB (8 .. 120, read once) sets the chunk size of both
- * two-pass schedules. */
+ * GBNTT_FOURSTEP_CHUNK_MB (8 .. 120, read once) takes the polynomials through
+ * both passes in chunks of that many MiB (default: all at once). */
 int gbntt_execute(const gbntt_plan* plan, const void* d_in, void* d_out, uint64_t batch,
                   void* stream);
 

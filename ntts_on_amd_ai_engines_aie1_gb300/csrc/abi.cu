@@ -136,9 +136,9 @@ int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, c
         g_launches.fetch_add((unsigned long long)nl, std::memory_order_relaxed);
         return GBNTT_OK;
     } else if (p->large.cols && batch <= p->two_pass_max) {
-        // two passes per chunk of polynomials; a chunk (large_chunk_bytes())
-        // stays in L2 between its passes.  Forward: columns then rows; inverse:
-        // rows first.  Programmatic dependent launches (grid_dep_start).
+        // two passes per chunk of polynomials (large_chunk_bytes()).  Forward:
+        // columns then rows; inverse: rows first.  Programmatic dependent
+        // launches (grid_dep_start).
         const LargeInfo& li = p->large;
         const long long n = (long long)p->hp.n;
         long long chunk = large_chunk_bytes() / (n * 4);

@@ -1261,6 +1261,11 @@ KernelInfo kinfo_r8(int L, bool lat);
 // canonical families (kernels_c16.cu, kernels_c32.cu)
 KernelInfo kinfo_canon(int fam, int L, bool lat);
 
+// The block of a pass: the second pass goes from the end to the beginning, so it
+// finds what the first one wrote last in L2 (2^26 coefficients, forward / inverse:
+// canonical 2^16 202/193 -> 200/190 us, 2^20 240/230 -> 237/225).
+__device__ __forceinline__ unsigned pass_block(bool first) { return first ? blockIdx.x : gridDim.x - 1 - blockIdx.x; }
+
 // two-pass schedule for int32 transforms longer than one CTA holds (kernels_large.cu)
 struct LargeInfo {
     const void* cols = nullptr;   // column pass kernel
@@ -1303,9 +1308,13 @@ cudaError_t launch_kernel(const void* fn, unsigned grid, int threads, int smem, 
 // 4 x 2^16 15.0 -> 11.0, of 1 x 2^20 23.2 -> 19.1; long calls within 1 %; the units
 // 173.8 -> 160.3 us over 2^26 coefficients (50 %: 163.3, 80 %: 165.5).
 constexpr int SMEM_SHARE = 60;
-// the polynomials of a call go through the two passes of the long int32
-// transforms in chunks of at most this many bytes, so the intermediate stays
-// in L2 (96 MiB; GBNTT_FOURSTEP_CHUNK_MB, 8 .. 120, read once per process)
+// A call's polynomials go through the two passes of the long int32 transforms in
+// chunks of at most this many bytes: all at once, unless GBNTT_FOURSTEP_CHUNK_MB
+// (8 .. 120, read once per process) says otherwise.  Chunks that stay in L2 save
+// the intermediate's trip through HBM, but the passes are bound by arithmetic,
+// and each of them starts and ends with a part of the chip idle.  2^28
+// coefficients (1 GiB), chunks of 96 MiB / 256 MiB / all at once, us for 2^26:
+// canonical 2^16 217 / 202 / 195, 2^20 308 / 282 / 271, lanes 2^20 451 / 433 / 427.
 long long large_chunk_bytes();
 
 // single-purpose kernels (kernels_misc.cu)

@@ -15,8 +15,7 @@
 // in which its threads read them (the tail: 16 coalesced bytes a lane).
 // The inverse (bit-reversed in, natural out, no n^-1) undoes the layers from the
 // low bits up (Gentleman-Sande, root^-bitrev(block)): rows, then columns.
-// Polynomials go through both passes in chunks of at most large_chunk_bytes(), so the
-// intermediate stays in L2 between the passes.
+// Polynomials go through both passes in chunks of at most large_chunk_bytes().
 //
 // The column pass moves 2D tiles (COLS adjacent columns x n1 rows) between
 // global and shared memory with the Tensor Memory Accelerator
@@ -29,10 +28,13 @@
 // multiply pipe for 7.6 clocks a warp, 56 % of a 2^12 row pass; its loads and
 // exchanges share the other half with the additions.  Over 2^26 coefficients,
 // forward / inverse, against the four-step that multiplies by a twist between
-// the passes (one factor per coefficient up to 2^20, two beyond):
+// the passes (one factor per coefficient up to 2^20, two beyond), in chunks of 96
+// MiB:
 //   2^16 224/229 -> 224/214 us    2^18 237/239 -> 230/224
 //   2^20 275/264 -> 265/256       2^22 317/322 -> 314/313
-// Without the tail (64 contiguous bytes a lane): 2^16 236/225, 2^20 269/264.
+// Without the tail (64 contiguous bytes a lane): 2^16 236/225, 2^20 269/264.  All
+// at once (large_chunk_bytes, pass_block): 2^16 200/190, 2^18 205/196, 2^20
+// 237/225, 2^22 280/274.
 #include <cuda.h>
 
 #include "canon_tables.h"
@@ -76,7 +78,7 @@ __global__ void __launch_bounds__(COLS << (L1 - EL))
     unsigned long long* bar = reinterpret_cast<unsigned long long*>(csm + N1 * COLS * 4);
     const int tid = threadIdx.x, cl = tid % COLS, g = tid / COLS;
     const long long tpp = n2 / COLS;                           // column tiles per polynomial
-    const long long t = tile0 + blockIdx.x;
+    const long long t = tile0 + pass_block(FWD);
     const int c0 = (int)((t % tpp) * COLS);
     const int r0 = (int)((t / tpp) * N1);
     if (tid == 0) {
@@ -138,7 +140,7 @@ __global__ void __launch_bounds__(1 << (L2 - EL), rows_min_blocks(L2, EL))
     extern __shared__ int rsm[];
     grid_dep_start();
     const int g = threadIdx.x;
-    const long long row = row0 + blockIdx.x;
+    const long long row = row0 + pass_block(!FWD);
     const int r = (int)(row & ((1 << L1) - 1));
     int v[E];
     if constexpr (FWD) {

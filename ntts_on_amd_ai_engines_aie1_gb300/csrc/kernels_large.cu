@@ -40,8 +40,9 @@ __global__ void __launch_bounds__(COLS << (L1 - large_el(L1)), kntt_min_blocks(F
     grid_dep_start();
     const int tid = threadIdx.x, cl = tid % COLS, g = tid / COLS;
     const long long blocks_per_poly = (1LL << L2) / COLS;
-    const long long poly = blockIdx.x / blocks_per_poly;
-    const long long c0 = (blockIdx.x % blocks_per_poly) * COLS;
+    const long long block = pass_block(topdown(FAM));
+    const long long poly = block / blocks_per_poly;
+    const long long c0 = (block % blocks_per_poly) * COLS;
     const long long base = (poly << (L1 + L2)) + c0 + cl;
     const int* in = static_cast<const int*>(a.in) + base;
     int* out = static_cast<int*>(a.out) + base;
@@ -65,7 +66,7 @@ __global__ void __launch_bounds__(P << (L2 - LARGE_EL), kntt_min_blocks(FAM, P <
     extern __shared__ int rsmem[];
     grid_dep_start();
     const int tid = threadIdx.x, lp = tid / G, g = tid % G;
-    const long long row = (long long)blockIdx.x * P + lp;        // rows of all polynomials, in order
+    const long long row = (long long)pass_block(!topdown(FAM)) * P + lp;        // rows of all polynomials, in order
     const bool active = row < (a.batch << L1);
     const int hi = (int)(row & ((1LL << L1) - 1));               // row index inside its polynomial
     int* sp = rsmem + lp * xwords(L2);

@@ -310,8 +310,8 @@ cudaError_t launch_kernel(const void* fn, unsigned grid, int threads, int smem, 
 long long large_chunk_bytes() {
     static const long long v = [] {
         const char* e = std::getenv("GBNTT_FOURSTEP_CHUNK_MB");
-        const long long x = e ? std::atoll(e) : 96;
-        return (x >= 8 && x <= 120 ? x : 96) << 20;
+        const long long x = e ? std::atoll(e) : 0;
+        return x >= 8 && x <= 120 ? x << 20 : 1LL << 62;
     }();
     return v;
 }
