@@ -128,8 +128,9 @@ int gbntt_plan_destroy(gbntt_plan* plan);
 
 /* Transforms `batch` polynomials held in device memory, asynchronously on
  * `stream` (a cudaStream_t; NULL = legacy default stream).  One kernel launch
- * per call, except the int32 designs with n >= 2^15 (up to 2^22), and with
- * n = 2^14 up to half a polynomial per SM, which run two passes (column and row
+ * per call, except the int32 designs with n >= 2^15 (up to 2^22), the canonical
+ * inverse of n = 2^14 and the others of n = 2^14 up to half a polynomial per SM,
+ * which run two passes (column and row
  * sub-transforms; the canonical column pass moves 2D tiles with the Tensor
  * Memory Accelerator).
  * In natural order n = 2^14 and 2^15 run one CTA per polynomial.  The

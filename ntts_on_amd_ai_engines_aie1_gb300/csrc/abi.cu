@@ -103,14 +103,17 @@ int sm_count() {
 // one CTA per polynomial, 2^16 and more do not.  One CTA takes the same time
 // for 1 polynomial as for 152 and keeps half an SM's threads waiting at its
 // barriers; two passes spread a polynomial over 16 .. 64 CTAs.  Measured (us,
-// one CTA -> two passes; 1 / 76 / 152 / 2^26 n^-1 polynomials):
-//   canonical 2^14  15.0 / 15.0 / 17.0 / 193 -> 10.9 / 14.0 / 17.0 / 210
-//   canonical 2^15  21.1 / 23.2 / 25.2 / 240 -> 10.9 / 18.0 / 25.2 / 218
-//   lanes 2^14      18.0 / 19.0 / 19.1 / 302 -> 10.9 / 16.0 / 21.1 / 324
-//   lanes 2^15      33.4 / 33.4 / 35.5 / 388 -> 10.9 / 22.1 / 33.4 / 343
-// so 2^15 always takes two passes and 2^14 up to half a polynomial per SM.  GBNTT_FOURSTEP_MIN_L (14 .. 16, read once per process) instead runs
-// canonical lengths from 2^that on in two passes and shorter ones in one CTA.
-uint64_t two_pass_limit(int L, bool canon) {
+// one CTA -> two passes; 1 / 76 / 152 / 1024 / 2^26 n^-1 polynomials):
+//   canonical 2^14 forward  15.0 / 15.0 / 17.0 / 58 / 193 -> 10.9 / 12.9 / 17.0 / 59 / 204
+//   canonical 2^14 inverse  15.0 / 15.0 / 17.0 / 60 / 197 -> 8.8 / 11.9 / 16.0 / 54 / 189
+//   canonical 2^15          21.1 / 23.2 / 25.2 / 127 / 240 -> 10.9 / 17.0 / 25.2 / 107 / 197
+//   lanes 2^14              18.0 / 19.0 / 19.1 / 85 / 302 -> 10.9 / 16.0 / 21.1 / 88 / 323
+//   lanes 2^15              33.4 / 33.4 / 35.5 / 196 / 388 -> 10.9 / 22.1 / 33.4 / 168 / 321
+// so 2^15 and the canonical inverse of 2^14 always take two passes and the
+// others of 2^14 up to half a polynomial per SM.  GBNTT_FOURSTEP_MIN_L (14 .. 16,
+// read once per process) instead runs canonical lengths from 2^that on in two
+// passes and shorter ones in one CTA.
+uint64_t two_pass_limit(int L, bool canon, bool inverse) {
     static const int env = [] {
         const char* e = std::getenv("GBNTT_FOURSTEP_MIN_L");
         const int x = e ? std::atoi(e) : 0;
@@ -119,7 +122,7 @@ uint64_t two_pass_limit(int L, bool canon) {
     if (L < 14) return 0;
     if (L >= 16) return UINT64_MAX;
     if (canon && env) return L >= env ? UINT64_MAX : 0;
-    return L == 15 ? UINT64_MAX : (uint64_t)(sm_count() / 2);
+    return L == 15 || (canon && inverse) ? UINT64_MAX : (uint64_t)(sm_count() / 2);
 }
 
 int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, cudaStream_t s) {
@@ -310,7 +313,7 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
     p->fam = canon ? canonical_family(kind) : family_of(kind);
     p->br = !canon && (kind == K_R4_I16_INV);
     if (p->fam >= 0 && hp.elem_bytes == 4 && !(flags & FLAG_NATURAL_ORDER))   // two passes have no natural-order form
-        p->two_pass_max = two_pass_limit(hp.L, canon);
+        p->two_pass_max = two_pass_limit(hp.L, canon, kind == K_R2_I32_INV);
     bool found = true;
     if (p->two_pass_max) {
         if (canon) p->clarge = canon_large_info(p->fam, hp.L);
