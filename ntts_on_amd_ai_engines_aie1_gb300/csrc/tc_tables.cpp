@@ -14,8 +14,7 @@ uint32_t f16_bits(int v) {
     if (!v) return 0;
     const uint32_t sign = v < 0 ? 0x8000u : 0u;
     uint32_t m = (uint32_t)(v < 0 ? -v : v);
-    int e = 31;
-    while (!((m >> e) & 1u)) --e;
+    const int e = 31 - __builtin_clz(m);
     return sign | (uint32_t)(e + 15) << 10 | ((e <= 10 ? m << (10 - e) : m >> (e - 10)) & 0x3FFu);
 }
 
@@ -101,6 +100,21 @@ void tc_build(int L, int64_t modulus, int64_t root, bool inverse, bool natural, 
     uint32_t* A = out.data();
     uint32_t* B = A + (size_t)tc_a_words(M.LK) * 4;
     uint32_t* W = B + (size_t)tc_b_words(M.LK) * 4;
+    // the index maps of all columns and rows once
+    int cp[32], cc[32], mr[16];
+    for (int i = 0; i < 8 * NT; ++i) M.col(i >> 3, i & 7, &cp[i], &cc[i]);
+    for (int i = 0; i < 16; ++i) mr[i] = M.m(i);
+    // a matrix entry's limbs, from its exponent: of 256 w and of w
+    struct Pair {
+        Limbs hi, lo;
+    };
+    std::vector<Pair> la(n), lb(n);
+    for (uint32_t e = 0; e < n; ++e) {
+        const uint32_t w = pw[e], w256 = w * 256 % q;
+        if (e % M.R2 == 0) la[e] = {limbs(w256, q, 2), limbs(w, q, 2)};
+        if (e % M.R1 == 0) lb[e] = {limbs(w256, q, 512), limbs(w, q, 512)};
+    }
+    const Limbs zero = {0, 0};
     for (int lane = 0; lane < 32; ++lane) {
         const int g = lane >> 2, t = lane & 3;
         // stage 1, A operand: h(256 W), h(W), l(256 W), l(W)
@@ -109,9 +123,9 @@ void tc_build(int L, int64_t modulus, int64_t root, bool inverse, bool natural, 
                 const int row = g + 8 * (r & 1), k0 = 2 * t + 8 * (r >> 1);
                 Limbs hi[2], lo[2];
                 for (int e = 0; e < 2; ++e) {
-                    const uint32_t w = power(M.m(row) * M.u(s, k0 + e) * M.R2);
-                    hi[e] = limbs(w * 256 % q, q, 2);
-                    lo[e] = limbs(w, q, 2);
+                    const Pair& x = la[(uint32_t)(mr[row] * M.u(s, k0 + e) * M.R2) & (n - 1)];
+                    hi[e] = x.hi;
+                    lo[e] = x.lo;
                 }
                 const uint32_t word[4] = {hi[0].h | hi[1].h << 16, lo[0].h | lo[1].h << 16, hi[0].l | hi[1].l << 16,
                                           lo[0].l | lo[1].l << 16};
@@ -125,12 +139,10 @@ void tc_build(int L, int64_t modulus, int64_t root, bool inverse, bool natural, 
                 for (int r = 0; r < 2; ++r) {
                     Limbs hi[2], lo[2];
                     for (int e = 0; e < 2; ++e) {
-                        const int k = 2 * t + 8 * r + e;
-                        int pc, c;
-                        M.col(2 * s + (k >> 3), k & 7, &pc, &c);
-                        const uint32_t w = pc == po ? power(c * v * M.R1) : 0u;
-                        hi[e] = limbs(w * 256 % q, q, 512);
-                        lo[e] = limbs(w, q, 512);
+                        const int k = 16 * s + 2 * t + 8 * r + e;
+                        const Pair& x = lb[(uint32_t)(cc[k] * v * M.R1) & (n - 1)];
+                        hi[e] = cp[k] == po ? x.hi : zero;
+                        lo[e] = cp[k] == po ? x.lo : zero;
                     }
                     uint32_t* h = B + (((s * 2 + jj) * 2 + 0) * 32 + lane) * 4;
                     uint32_t* l = B + (((s * 2 + jj) * 2 + 1) * 32 + lane) * 4;
@@ -144,9 +156,7 @@ void tc_build(int L, int64_t modulus, int64_t root, bool inverse, bool natural, 
         for (int j = 0; j < NT; ++j)
             for (int p = 0; p < S1; ++p)
                 for (int i = 0; i < 4; ++i) {
-                    int po, c;
-                    M.col(j, 2 * t + (i & 1), &po, &c);
-                    const int m = M.m(g + 8 * (i >> 1)) + 16 * p;
+                    const int c = cc[8 * j + 2 * t + (i & 1)], m = mr[g + 8 * (i >> 1)] + 16 * p;
                     const uint32_t w = power(m * c) * fac % q;
                     uint32_t* d = W + (((j * S1 + p) * 2 + (i >> 1)) * 32 + lane) * 4 + 2 * (i & 1);
                     const uint32_t hi = (w << 16) / q;
