@@ -290,7 +290,7 @@ def run_ours(args):
     torch.cuda.synchronize()
     launches0 = gb.launch_count()
     t_wall0 = time.time()
-    # one plain launch of the persistent kernel per step (a CUDA graph replay of
+    # one plain launch of the batch kernel per step (a CUDA graph replay of
     # the same single launch measured 0.9-1.2 us slower per step; see run)
     step_ms = timed(lambda: batch.execute(stream), args.steps)
     t_wall1 = time.time()
@@ -381,13 +381,13 @@ def run_ours(args):
         "vs_baseline": None, "dtype": "int16", "data": "synthetic",
         "config": workload_config(args.arith, world),
         "coefficients_per_s": value * coeffs_per_poly(),
-        "run": {"launch": "one persistent kernel launch per step (gbntt_batch_execute)", "arithmetic": args.arith,
+        "run": {"launch": "one batch kernel launch per step (gbntt_batch_execute)", "arithmetic": args.arith,
                 "graph_replay_ms_per_step": graph_ms,
                 "autotuned_log2_coeffs_per_thread": batch.query(4), "autotuned_cta_threads": batch.query(6),
                 "autotuned_ctas_per_sm_budget": batch.query(7)},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": peak_src,
-                     "kernel": f"k_batch<int16> persistent radix-4 ({args.arith} arithmetic, all 16384 polys "
+                     "kernel": f"the int16 batch kernel of the autotuner's choice ({args.arith} arithmetic, all 16384 polys "
                                "per launch)",
                      "algorithmic_bytes_per_launch": algo_bytes, "avg_launch_ms": ms,
                      "traffic": tr.get("bytes_per_launch"),
@@ -415,11 +415,11 @@ def run_configs(gb, oracle, flush, stream, peak, arith):
       C3 twin: the headline batch in the other arithmetic;
       C1: radix-2 int16 forward then inverse, n = 1024, one polynomial (latency);
       C2: radix-2 int32 forward + inverse, n = 4096, 1024 polynomials for each
-          of four primes (one persistent launch per direction);
+          of four primes (one batch launch per direction);
       C4a: ragged radix-8 int16 forward with the bit reversal fused, 2000
-          polynomials of n = 2^U, U uniform in {8..12}, one persistent launch;
+          polynomials of n = 2^U, U uniform in {8..12}, one batch launch;
       C4b: int32 forward and inverse of 64 polynomials of n = 2^20, q = 998244353
-          (canonical: the TMA-fed four-step; lanes: the two-pass schedule);
+          (canonical: the TMA-fed two passes; lanes: the two-pass schedule);
       C16k: int32 forward and inverse of 4096 polynomials of n = 2^14.
     Entries for n >= 2^14 carry a roofline object like the headline's."""
     import torch
@@ -493,7 +493,7 @@ def run_configs(gb, oracle, flush, stream, peak, arith):
         ms = timed(lambda: (f.execute(dx, y, 1, stream), i.execute(y, z, 1, stream)), 200)
         out[f"C1_r2_i16_fwd_inv_n1024_{name}"] = {"us_per_fwd_inv_pair": ms * 1e3, "launches": 2}
 
-    # C2: the four primes' forward transforms as one persistent launch, then the inverses
+    # C2: the four primes' forward transforms as one batch launch, then the inverses
     n, cnt = 4096, 1024
     for name, fl in (("canonical", CAN), ("lanes", 0)):
         fwd_segs, inv_segs, keep = [], [], []
@@ -519,7 +519,7 @@ def run_configs(gb, oracle, flush, stream, peak, arith):
         out[f"C2_r2_i32_fwd_inv_n4096_4primes_{name}"] = entry(8 * cnt, 8 * cnt * n, nb, ms, 2)
         del bf, bi, fwd_segs, inv_segs
 
-    # C4a: ragged radix-8, natural-order output, one persistent launch
+    # C4a: ragged radix-8, natural-order output, one batch launch
     q = 12289
     U = rng.integers(8, 13, 2000)
     for name, fl in (("canonical", CAN), ("lanes", 0)):
@@ -583,8 +583,8 @@ def run_configs(gb, oracle, flush, stream, peak, arith):
                 key = f"{tag}_r2_i32_{d}_n2^{L}_{cnt}_{name}"
                 out[key] = entry(cnt, cnt * n, nb, ms, launches)
                 if fl:
-                    kern = ("four-step: k_ccols (TMA column pass) + k_crows (twist, row pass)" if L >= 16
-                            else "k_ntt (one CTA per polynomial)")
+                    kern = ("two passes: k_ccols (TMA column pass) + k_crows (row pass)" if L >= 16
+                            else "k_ntt (one CTA per polynomial; the inverse in two passes)")
                     out[key]["roofline"] = roofline(key, nb, ms, kern)
     return out
 
@@ -720,7 +720,7 @@ PROFILE_CASES = {
     "bitrev_4096": (6, 4096, 12289, 0, 65536),
     "fullbarrett_4096": (7, 4096, 12289, 0, 65536),
     "r8stage_4096": (3, 4096, 12289, 41, 65536),
-    "batch_r4": None,   # the benchmark batch, 4x larger, persistent kernel
+    "batch_r4": None,   # the benchmark batch, 4x larger, batch kernel
     "c_batch_r4": None,  # the same with GBNTT_FLAG_CANONICAL
 }
 

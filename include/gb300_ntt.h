@@ -177,14 +177,18 @@ int gbntt_plan_query(const gbntt_plan* plan, int what, int64_t* value);
 int gbntt_host_tables(int kind, uint32_t n, int64_t q, int64_t root, int64_t factor,
                       uint32_t flags, int which, int64_t* dst, int64_t cap, int64_t* len);
 
-/* ---- batches: many polynomials of several designs in one persistent launch ----
+/* ---- batches: many polynomials of several designs in one launch ----
  *
  * A batch is a fixed list of segments (plan, device input, device output,
  * number of polynomials).  gbntt_batch_execute transforms all of them with one
- * persistent kernel launch per storage type (int16 designs, int32 designs):
- * tiles of polynomials are handed out dynamically, largest n first, and move
- * between HBM and shared memory as bulk (TMA) copies, double-buffered.
- * Segments the persistent kernel does not cover (bit-reversal, full Barrett,
+ * kernel launch per storage type and arithmetic (int16 or int32, lanes or
+ * canonical), of the fastest of three kernels: the persistent one (tiles of
+ * polynomials are handed out dynamically, largest n first, and move between
+ * HBM and shared memory as bulk (TMA) copies, double-buffered), the direct one
+ * (a CTA per tile, coefficients straight to registers) and, for canonical
+ * int16 batches of n = 2^5 .. 2^10, the tensor-core one.  The direct and the
+ * tensor-core launch are programmatic dependent launches, like the plans'.
+ * Segments the batch kernels do not cover (bit-reversal, full Barrett,
  * the radix-8 single stage, the radix-4 inverse, in-place segments, n outside
  * its range) run as their plans' own launches after it, on the same stream.
  * The batch owns a few words of device scratch (tile counter), so launches of
@@ -198,10 +202,11 @@ typedef struct gbntt_segment {
 
 typedef struct gbntt_batch gbntt_batch;
 
-/* flags: GBNTT_BATCH_NO_TUNE skips the autotuner, which otherwise times every
- * persistent-kernel configuration (coefficients per thread, hence threads
+/* flags: GBNTT_BATCH_NO_TUNE skips the autotuner, which otherwise times the
+ * configurations of the three kernels (coefficients per thread, hence threads
  * and CTAs per transform and polynomials per tile, and resident CTAs per SM)
- * on the batch itself at creation and keeps the fastest.  A batch whose
+ * on the batch itself at creation and keeps the fastest; those that fall
+ * behind are dropped between its rounds.  A batch whose
  * inputs and outputs fit in L2 is timed from HBM: creation then briefly
  * allocates twice the L2 size of scratch to evict it between the timed
  * launches (without room for it, the launches are timed back to back).
@@ -236,13 +241,14 @@ int gbntt_batch_status(gbntt_batch* batch);
  * A tile whose wait runs out makes its CTA record GBNTT_ERR_TIMEOUT (reported
  * by gbntt_batch_status, gbntt_noalloc_status and the server's waits), let its
  * copies in flight land (those waits keep the default limit) and stop.  Small
- * limits are for tests of that failure path.  No counterpart in the reference
+ * limits are for tests of that failure path; while one is set, batches run the
+ * persistent kernel (the other two have no such waits).  No counterpart in the reference
  * (AIE graphs have no runtime error channel). */
 #define GBNTT_WAIT_POLLS_DEFAULT 4194304u
 int gbntt_set_wait_limit(uint32_t polls);
 #define GBNTT_BQ_LAUNCHES 0   /* kernel launches per execute            */
-#define GBNTT_BQ_TILES    1   /* tiles of the persistent launches        */
-#define GBNTT_BQ_GRID     2   /* CTAs of the largest persistent launch   */
+#define GBNTT_BQ_TILES    1   /* tiles of the batch kernels' launches    */
+#define GBNTT_BQ_GRID     2   /* CTAs of the largest of these launches   */
 #define GBNTT_BQ_SMEM     3   /* dynamic shared memory per CTA (bytes)   */
 #define GBNTT_BQ_EL16     4   /* log2 coefficients per thread chosen for the int16 launch */
 #define GBNTT_BQ_FAMSET   5   /* design families compiled into the chosen int16 kernel (bit mask) */
@@ -252,8 +258,9 @@ int gbntt_set_wait_limit(uint32_t polls);
 /* Setting the environment variable GBNTT_TUNE_LOG=1 prints the autotuner's
  * timing of every candidate configuration to stderr at batch creation;
  * GBNTT_TUNE_FORCE="<log2 coefficients per thread>,<CTAs per SM, 0 = default>"
- * pins the choice among the candidates (the timing launches still run), "tc"
- * the tensor-core kernel (canonical int16 batches of n = 2^5 .. 2^10). */
+ * pins the choice among the persistent kernel's candidates (the timing launches
+ * still run), "d<threads per CTA>,<log2 coefficients per thread>" among the
+ * direct kernel's, "tc" the tensor-core kernel. */
 int gbntt_batch_query(const gbntt_batch* batch, int what, int64_t* value);
 int gbntt_batch_destroy(gbntt_batch* batch);
 

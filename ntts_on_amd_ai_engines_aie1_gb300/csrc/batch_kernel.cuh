@@ -1,5 +1,6 @@
 // batch_kernel.cuh -- the persistent batch kernel template (instantiated in
-// batch_k16.cu and batch_k32.cu, launched by batch.cu).
+// batch_k16.cu and batch_k32.cu, launched by batch.cu), one of the three batch
+// kernels: batch_direct.cuh and tc16.cuh have the others.
 #pragma once
 
 #include "persist.cuh"

@@ -41,14 +41,16 @@ enum Fam {
 __host__ __device__ constexpr bool fam_canon(int fam) { return fam >= F_C16F && fam <= F_C32I; }
 
 // Programmatic dependent launch.  The library's per-plan launches (every
-// design's kernel, the two passes of a long transform and its chunks; not the
-// persistent batch kernels) carry the programmatic-stream-serialization
+// design's kernel, the two passes of a long transform) and the direct and
+// tensor-core batch launches (not the persistent one, whose tile counter is
+// re-armed by its last CTA) carry the programmatic-stream-serialization
 // attribute, so when the previous operation is a grid that has signalled
 // launch_dependents, their CTAs take the SM slots its last CTAs free, with no
 // launch gap.  Every such kernel starts with grid_dep_start(): it signals its
 // own dependents (safe this early: their wait covers this whole grid and its
 // memory operations) and waits for the previous grid's completion and results
-// before touching global memory.  After any other operation, or without the
+// before touching global memory (but the plan's tables, which never change).
+// After any other operation, or without the
 // attribute, the launch is ordered as usual and both instructions are no-ops.
 __device__ __forceinline__ void grid_dep_start() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
