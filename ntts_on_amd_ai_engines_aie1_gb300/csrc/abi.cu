@@ -190,8 +190,16 @@ int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, c
         // measured 6-8 % slower for int32 and radix-8).
         const int sms = sm_count();
         const bool small = batch <= (uint64_t)sms;
-        if (p->tc_fn) {
-            const unsigned long long tiles = ((batch << p->hp.L) + TC_TILE - 1) / TC_TILE;
+        // The tensor-core form from more than two tiles (of 1024 coefficients) per
+        // SM: a warp takes a whole tile, so with fewer the window kernel spreads
+        // over more threads.  n = 32, where two thirds of the matrix products are
+        // with zeros, stays with the window kernel.  Forward + inverse after an L2
+        // flush, us, window / tensor cores: 1024 x 1 8.9 / 10.9, x 152 9.4 / 10.9,
+        // x 304 10.9 / 10.9, x 608 12.3 / 12.3, x 4864 25.2 / 22.0; 256 x 8 9.2 /
+        // 10.3, x 1216 10.1 / 10.9, x 4864 11.8 / 10.9, x 19456 21.1 / 20.6;
+        // 32 x 155648 18.6 / 20.8.
+        const unsigned long long tiles = ((batch << p->hp.L) + TC_TILE - 1) / TC_TILE;
+        if (p->tc_fn && tiles > 2ull * (unsigned)sms) {
             // a warp per tile; one-warp CTAs, which spread over the SMs, up to
             // the resident count
             const unsigned long long cap = (unsigned long long)TC_OCC * (unsigned)sms;
@@ -465,7 +473,7 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
             a.tctab = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(p->d_tab) + p->tab_bytes);
             a.tc_ke = (int)tc_ke;
             a.tc_corr = (int)tc_corr;
-            p->tc_fn = tc16_kernel(hp.L, inverse && !natural, !inverse && !natural);
+            if (hp.L > TC_MIN_L) p->tc_fn = tc16_kernel(hp.L, inverse && !natural, !inverse && !natural);
         }
     }
     a.natural_in = ((flags & FLAG_NATURAL_ORDER) && inverse) ? 1 : 0;

@@ -145,3 +145,24 @@ def test_radix8_stage_over_many_polynomials(gb, n, count):  # noqa: F811
     stride = torch.cuda.get_device_properties(0).multi_processor_count * 32 * 128 // max(1, n // 16)
     for lo in (0, min(stride, count) - 8, count - 9):
         assert torch.equal(y[lo:lo + 9], plan(x[lo:lo + 9].clone())), lo
+
+
+@pytest.mark.parametrize("L", [5, 6, 7, 8, 9, 10])
+@pytest.mark.parametrize("kind,flags", [(0, 1), (0, 9), (1, 1), (1, 9), (1, 17)])
+def test_window_and_tensor_core_forms(gb, L, kind, flags):  # noqa: F811
+    """A canonical int16 call changes from the window kernel to the tensor
+    cores behind two tiles of 1024 coefficients per SM (one-warp CTAs up to
+    four, then larger ones): calls with a few coefficients in their last tile
+    on both sides of both lines equal the calls on their parts, which stay with
+    the window kernel."""
+    n, q = 1 << L, 12289
+    root = next(r for g in range(2, q) if pow(r := pow(g, (q - 1) >> L, q), n >> 1, q) == q - 1)
+    plan = gb.Plan(kind, n, q, root, 0, flags)
+    sms, tile = torch.cuda.get_device_properties(0).multi_processor_count, 1024 // n
+    line = 2 * sms * tile                       # the largest call of the window kernel
+    g = torch.Generator(device="cuda").manual_seed(SEED + L)
+    for count in (line, line + 1, 4 * sms * tile - tile + 1, 4 * sms * tile + 1):
+        x = torch.randint(-32768, 32768, (count, n), generator=g, device="cuda", dtype=torch.int16)
+        want = torch.cat([plan(x[:line // 2].contiguous()), plan(x[line // 2:line].contiguous())]
+                         + [plan(x[i:i + line].contiguous()) for i in range(line, count, line)])
+        assert torch.equal(plan(x), want), count
