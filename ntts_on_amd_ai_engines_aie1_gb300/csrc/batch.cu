@@ -560,7 +560,7 @@ int gbntt_batch_execute_host(gbntt_batch* b, const void* const* h_in, void* cons
         return (size_t)u.count * (size_t)n * (size_t)eb;
     };
     // Zero copy: when every batched segment's host buffers are page-locked and
-    // mapped, one k_batch_zc launch per storage type reads and writes them in
+    // mapped, one k_batch_zc launch per part reads and writes them in
     // place, so inbound and outbound traffic overlap on the host-device link
     // instead of running as two copy phases.  Segments outside the persistent
     // kernel still go through their device buffers.
@@ -574,7 +574,7 @@ int gbntt_batch_execute_host(gbntt_batch* b, const void* const* h_in, void* cons
                     !((reinterpret_cast<uintptr_t>(mi) | reinterpret_cast<uintptr_t>(mo)) & 15);
     }
     if (zero_copy) {
-        std::vector<SegDev> uploaded[2];   // committed as the live descriptors once the call completed
+        std::vector<SegDev> uploaded[BATCH_PARTS];   // committed as the live descriptors once the call completed
         for (int i = 0; i < b->nparts; ++i) {
             auto& part = b->parts[i];
             auto& lay = part.zlay;
