@@ -131,10 +131,15 @@ int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, c
     a.out = d_out;
     a.batch = (long long)batch;
     cudaError_t e = cudaSuccess;
+    // a call whose grid would not fit one launch is refused, whatever form it takes
+    auto too_large = [&](unsigned long long blocks_per_poly) { return batch > 0x7FFFFFFFull / blocks_per_poly; };
     if (p->clarge.cols && batch <= p->two_pass_max) {
+        const CanonLarge& li = p->clarge;
+        if (too_large(std::max(1ull << li.L1, (1ull << li.L2) / li.cols_width)))
+            return fail(GBNTT_ERR_ARG, "batch too large for one launch");
         const bool inverse = (p->hp.kind == K_R2_I32_INV);
         int nl = 0;
-        e = launch_canon_large(p->clarge, a, p->tab_blocks, d_in, d_out, (long long)batch, inverse, p->d_err, s, &nl);
+        e = launch_canon_large(li, a, p->tab_blocks, d_in, d_out, (long long)batch, inverse, p->d_err, s, &nl);
         if (e != cudaSuccess) return cuda_fail(e, "two-pass launch");
         g_launches.fetch_add((unsigned long long)nl, std::memory_order_relaxed);
         return GBNTT_OK;
@@ -143,6 +148,8 @@ int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, c
         // columns then rows; inverse: rows first.  Programmatic dependent
         // launches (grid_dep_start).
         const LargeInfo& li = p->large;
+        if (too_large(std::max(1ull << li.L1, (1ull << li.L2) / li.cols_per_cta)))
+            return fail(GBNTT_ERR_ARG, "batch too large for one launch");
         const long long n = (long long)p->hp.n;
         long long chunk = large_chunk_bytes() / (n * 4);
         if (chunk < 1) chunk = 1;
@@ -190,6 +197,9 @@ int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, c
         // measured 6-8 % slower for int32 and radix-8).
         const int sms = sm_count();
         const bool small = batch <= (uint64_t)sms;
+        const KernelInfo& k = small && p->kl.fn ? p->kl : p->ki;
+        if (batch > 0x7FFFFFFFull * (unsigned)k.polys) return fail(GBNTT_ERR_ARG, "batch too large for one launch");
+        const unsigned long long blocks = (batch + k.polys - 1) / k.polys;
         // The tensor-core form from more than two tiles (of 1024 coefficients) per
         // SM: a warp takes a whole tile, so with fewer the window kernel spreads
         // over more threads.  n = 32, where two thirds of the matrix products are
@@ -212,9 +222,6 @@ int launch(const gbntt_plan* p, const void* d_in, void* d_out, uint64_t batch, c
             g_launches.fetch_add(1, std::memory_order_relaxed);
             return GBNTT_OK;
         }
-        const KernelInfo& k = small && p->kl.fn ? p->kl : p->ki;
-        const unsigned long long blocks = (batch + k.polys - 1) / k.polys;
-        if (blocks > 0x7FFFFFFFull) return fail(GBNTT_ERR_ARG, "batch too large for one launch");
         a.tab_bytes = blocks <= (unsigned long long)sms ? (int)p->tile_tab_bytes : 0;
         void* args[] = {&a};
         e = launch_kernel(k.fn, (unsigned)blocks, k.threads, k.smem, args, s, true);
