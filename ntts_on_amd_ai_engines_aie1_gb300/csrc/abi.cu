@@ -390,9 +390,9 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
     uint32_t tc_ke = 0, tc_corr = 0;
     if (canon) {
         // canonical families: (w, w') pairs computed on the device: the table
-        // of the whole transform where one CTA may run it (batches do, at
-        // every length that fits), then the block table of the two passes
-        const size_t n_tile = hp.L <= 15 ? canon_table_entries(hp.L, inverse) : 0;
+        // of the whole transform where one CTA runs any of the plan's calls,
+        // then the tables of the two passes
+        const size_t n_tile = p->two_pass_max != UINT64_MAX ? canon_table_entries(hp.L, inverse) : 0;
         const size_t n_blocks = p->clarge.cols ? two_pass_entries(hp.L) : 0;
         p->tile_tab_bytes = n_tile * sizeof(int2);
         p->tab_bytes = (n_tile + n_blocks) * sizeof(int2);
@@ -413,7 +413,7 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
         if (n_tile) e = make_canon_table(p->d_tab, hp.L, q32, (uint32_t)hp.root, inverse, 0);
         if (n_blocks) {
             p->tab_blocks = p->d_tab + n_tile;
-            if (e == cudaSuccess) e = 
+            if (e == cudaSuccess)
                 e = make_two_pass_tables(p->d_tab + n_tile, hp.L, p->clarge.L2, p->clarge.row_el, q32, (uint32_t)hp.root,
                                          inverse, 0);
             if (e == cudaSuccess) e = cudaMemsetAsync(p->d_err, 0, 256, 0);
