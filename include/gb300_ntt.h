@@ -119,7 +119,10 @@ typedef struct gbntt_plan gbntt_plan;
  * until gbntt_plan_destroy).  `root` is a primitive n-th root of unity modulo
  * q (the inverse designs invert it themselves, like src/twiddle.h:80,112).
  * `factor` is the multiplier of GBNTT_FULL_BARRETT_I16 (e.g. n^-1 mod q,
- * src/project.cpp:154); ignored otherwise.  BITREV_I16 ignores q and root. */
+ * src/project.cpp:154); ignored otherwise.  BITREV_I16 ignores q and root.
+ * A plan holds at most 8 n bytes of device memory for an int32 design (the
+ * canonical forward of 2^14: 16 n), so a canonical plan of 2^20 holds 8 MiB and
+ * one of 2^22 32 MiB; GBNTT_Q_TABLE_BYTES tells the size. */
 int gbntt_plan_create(gbntt_plan** plan, int kind, uint32_t n, int64_t q, int64_t root,
                       int64_t factor, uint32_t flags);
 

@@ -32,7 +32,7 @@ struct gbntt_plan {
     LargeInfo large;       // int32 n >= 2^14: two-pass schedule (large.cols != nullptr)
     CanonLarge clarge;     // canonical int32 n >= 2^14: two passes (clarge.cols != nullptr)
     uint64_t two_pass_max = 0;        // calls of more polynomials than this run one CTA per polynomial
-    const int2* tab_blocks = nullptr; // clarge: the block table (inside d_tab)
+    const int2* tab_blocks = nullptr; // clarge: the tables of the two passes (inside d_tab)
     unsigned* d_err = nullptr;        // clarge: set when a bounded wait ran out
     KArgs base;            // constants shared by every launch
     int2* d_tab = nullptr;
@@ -393,7 +393,7 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
         // of the whole transform where one CTA runs any of the plan's calls,
         // then the tables of the two passes
         const size_t n_tile = p->two_pass_max != UINT64_MAX ? canon_table_entries(hp.L, inverse) : 0;
-        const size_t n_blocks = p->clarge.cols ? two_pass_entries(hp.L) : 0;
+        const size_t n_blocks = p->clarge.cols ? two_pass_entries(hp.L, p->clarge.row_el) : 0;
         p->tile_tab_bytes = n_tile * sizeof(int2);
         p->tab_bytes = (n_tile + n_blocks) * sizeof(int2);
         if (hp.elem_bytes == 2 && tc_supported(hp.L, hp.q)) {

@@ -45,25 +45,34 @@ __global__ void k_canon_table(int2* tab, int L, unsigned q, unsigned root, int i
     }
 }
 
-// 2^(L-1) entries: entry b = root^(+-bitrev(b)), L - 1 bits reversed
-__global__ void k_block_table(int2* tab, int L, unsigned q, unsigned root, int inverse) {
-    const int n = 1 << L;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n / 2; i += gridDim.x * blockDim.x) {
-        unsigned long long e = __brev((unsigned)i) >> (33 - L);
+// the tail's words of the layer on bit 0, which hold every block's entry
+// (canon_tables.h): the right one of two neighbours is the left one times
+// root^(+-bitrev(1)) = root^(+-n/4)
+__global__ void k_tail_all(int4* tail, int L, int L2, int EL, unsigned q, unsigned root, int inverse) {
+    const int n = 1 << L, g2 = L2 - EL, w2 = EL - 2;          // log2 threads of a row, words of the layer
+    const unsigned quarter = powmod_dev(root, inverse ? 3u * (unsigned)(n / 4) : (unsigned)(n / 4), q);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n / 4; i += gridDim.x * blockDim.x) {
+        const int g = i & ((1 << g2) - 1), word = (1 << w2) - 1 + ((i >> g2) & ((1 << w2) - 1)), r = i >> (g2 + w2);
+        unsigned long long e = __brev((unsigned)two_pass_tail_block(L2, EL, r, word, g)) >> (33 - L);
         if (inverse && e) e = (unsigned long long)n - e;
-        tab[i] = shoup_pair(powmod_dev(root, e, q), q);
+        const unsigned w = powmod_dev(root, e, q);
+        const int2 x = shoup_pair(w, q), y = shoup_pair(mulmod(w, quarter, q), q);
+        tail[two_pass_tail_at(L2, EL, r, word, g)] = make_int4(x.x, x.y, y.x, y.y);
     }
 }
 
-// the tail (see canon_tables.h), from the block table
-__global__ void k_tail_table(int4* tail, const int2* tab, int L, int L2, int EL) {
-    const int g2 = L2 - EL;                                   // log2 threads of a row
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 1 << (L - 1); i += gridDim.x * blockDim.x) {
-        const int g = i & ((1 << g2) - 1), pair = (i >> g2) & ((1 << (EL - 1)) - 1), r = i >> (L2 - 1);
-        const int p = 31 - __clz(pair + 1), B = EL - 2 - p;   // 2^p pairs on bit B
-        if (B < 0) continue;                                  // the last word of each thread is unused
-        const int2* t = tab + ((((r << g2) | g) << (p + 1)) | 2 * (pair + 1 - (1 << p)));
-        tail[i] = make_int4(t[0].x, t[0].y, t[1].x, t[1].y);
+// the block table and the tail's other words, copied from those
+__global__ void k_two_pass_rest(int2* blocks, int4* tail, int L, int L2, int EL) {
+    const int g2 = L2 - EL, rest = (1 << (EL - 2)) - 1;       // words of the other layers
+    const long long nb = (long long)two_pass_blocks(L) / 2, count = nb + ((long long)rest << (L - EL));
+    for (long long i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        if (i < nb) {
+            reinterpret_cast<int4*>(blocks)[i] = tail[two_pass_tail_of(L2, EL, (int)(2 * i))];
+        } else {
+            const int j = (int)(i - nb), g = j & ((1 << g2) - 1), word = (j >> g2) % rest, r = (j >> g2) / rest;
+            tail[two_pass_tail_at(L2, EL, r, word, g)] =
+                tail[two_pass_tail_of(L2, EL, two_pass_tail_block(L2, EL, r, word, g))];
+        }
     }
 }
 
@@ -82,13 +91,12 @@ cudaError_t make_canon_table(int2* d_tab, int L, uint32_t q, uint32_t root, bool
     return cudaGetLastError();
 }
 
-size_t two_pass_entries(int L) { return ((size_t)1 << (L - 1)) + ((size_t)1 << L); }
-
 cudaError_t make_two_pass_tables(int2* d_tab, int L, int L2, int EL, uint32_t q, uint32_t root, bool inverse,
                                  cudaStream_t s) {
-    const int grid = grid_of(1ll << (L - 1));
-    k_block_table<<<grid, 256, 0, s>>>(d_tab, L, q, root, inverse ? 1 : 0);
-    k_tail_table<<<grid, 256, 0, s>>>(reinterpret_cast<int4*>(d_tab + ((size_t)1 << (L - 1))), d_tab, L, L2, EL);
+    int4* tail = reinterpret_cast<int4*>(d_tab + two_pass_blocks(L));
+    const int grid = grid_of(1ll << (L - 2));
+    k_tail_all<<<grid, 256, 0, s>>>(tail, L, L2, EL, q, root, inverse ? 1 : 0);
+    k_two_pass_rest<<<grid, 256, 0, s>>>(d_tab, tail, L, L2, EL);
     return cudaGetLastError();
 }
 

@@ -96,7 +96,7 @@ struct KArgs {
 // transformed (the matrices stay in parameter or shared memory).
 struct KC {
     const int2* tab;
-    const int4* tail;     // canonical two-pass rows: the thread's column of the tail table (canon_tables.h)
+    const int4* tail;     // canonical two-pass rows: the thread's words of the tail table (canon_tables.h)
     const int* tab16;
     const int* f8;
     const int* ftail;

@@ -9,10 +9,11 @@
 // n2 and the polynomial viewed as n1 rows of n2 coefficients (row-major, no
 // transpose in memory), the layers on the high bits are transforms of the
 // columns, the same for every column, and those on the low bits are transforms
-// of the rows, whose block index carries the row in its top bits.  One table of
-// n / 2 pairs serves all of them, and nothing is multiplied between the passes;
-// a row's entries for its lowest four bits are held a second time in the order
-// in which its threads read them (the tail: 16 coalesced bytes a lane).
+// of the rows, whose block index carries the row in its top bits.  One set of n / 2
+// pairs serves all of them, and nothing is multiplied between the passes.  A
+// row's entries for its lowest bits lie in the order in which its threads read
+// them (the tail: 16 coalesced bytes a lane); the block table needs the first n
+// / 8 pairs beside it, 8 bytes a coefficient together (canon_tables.h).
 // The inverse (bit-reversed in, natural out, no n^-1) undoes the layers from the
 // low bits up (Gentleman-Sande, root^-bitrev(block)): rows, then columns.
 // Polynomials go through both passes in chunks of at most large_chunk_bytes().
@@ -130,6 +131,15 @@ constexpr int rows_min_blocks(int L2, int el) {
     const int b = (L2 <= 10 ? 1024 : 1536) >> (L2 - el);
     return b > 16 ? 16 : b;
 }
+// every layer that reads the block table is on bit 2 or above: its blocks are
+// among the first n / 8
+constexpr bool rows_blocks_held(int fam, int L2, int el) {
+    for (int s = 0; s < nsteps(fam, L2); ++s) {
+        const int b = step_b(fam, L2, s), lo = window_lo(fam, L2, el, s);
+        if (b < 2 && (lo != 0 || b > el - 2)) return false;
+    }
+    return true;
+}
 template <int FAM, int L2, int EL>
 __global__ void __launch_bounds__(1 << (L2 - EL), rows_min_blocks(L2, EL))
     k_crows(const __grid_constant__ KArgs a, int L1, long long row0) {
@@ -137,6 +147,7 @@ __global__ void __launch_bounds__(1 << (L2 - EL), rows_min_blocks(L2, EL))
     constexpr int LO0 = window_lo(FAM, L2, EL, 0), LOZ = window_lo(FAM, L2, EL, NS - 1);
     constexpr bool FWD = topdown(FAM);
     static_assert((FWD ? LOZ : LO0) == 0, "contiguous runs at the rows' outer side");
+    static_assert(rows_blocks_held(FAM, L2, EL), "the block table is too short for this split");
     extern __shared__ int rsm[];
     grid_dep_start();
     const int g = threadIdx.x;
@@ -153,7 +164,7 @@ __global__ void __launch_bounds__(1 << (L2 - EL), rows_min_blocks(L2, EL))
         prologue<FAM>(v, a);                                   // raw input (the first pass)
     }
     KC kc = make_kc(a);
-    kc.tail = reinterpret_cast<const int4*>(a.tab + (1LL << (L1 + L2 - 1))) + ((long long)r << (L2 - 1)) + g;
+    kc.tail = reinterpret_cast<const int4*>(a.tab + two_pass_blocks(L1 + L2)) + two_pass_tail_at(L2, EL, r, 0, g);
     run_steps_x<FAM, L2, EL, 0, true>(v, rsm, g, kc, r, 0, std::make_integer_sequence<int, NS>{}, true);   // rsm untouched so far
     if constexpr (FWD) {
         epilogue<FAM, false>(v, a);                            // the forward's last pass

@@ -33,3 +33,7 @@ def test_canonical_reduction(tmp_path):
 
 def test_lane_rounding(tmp_path):
     _run_host_check(tmp_path, "lane_rounding")
+
+
+def test_two_pass_tables(tmp_path):
+    _run_host_check(tmp_path, "two_pass_tables")

@@ -24,3 +24,10 @@ def test_no_one_cta_table_where_every_call_takes_two_passes(gb):  # noqa: F811
         assert table_bytes(gb, kind, 15, 9) == 8 << 15 and table_bytes(gb, kind, 14, 9) == 8 << 14
     assert table_bytes(gb, 5, 14) * 4 == two
     assert table_bytes(gb, 4, 14) == table_bytes(gb, 5, 14) + (8 << 14)
+
+
+@pytest.mark.parametrize("L", [14, 15, 16, 18, 20, 22])
+def test_two_pass_tables_take_8_bytes_a_coefficient(gb, L):  # noqa: F811
+    for kind in (4, 5):
+        one_cta = 8 << L if (kind, L) == (4, 14) else 0
+        assert table_bytes(gb, kind, L) <= (8 << L) + one_cta
