@@ -381,6 +381,9 @@ int gbntt_batch_create(gbntt_batch** out, const gbntt_segment* segs, uint32_t ns
         part.fam_mask |= 1 << fam;
         part.pending.push_back({k, fam, L, eb, a});
     }
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // candidate configurations of each part: those whose family set covers it
     // and whose CTAs hold its longest transform
     for (int i = 0; i < b->nparts; ++i) {
@@ -407,17 +410,37 @@ int gbntt_batch_create(gbntt_batch** out, const gbntt_segment* segs, uint32_t ns
             gbntt_batch_destroy(b);
             return batch_fail(GBNTT_ERR_ARG, "no persistent kernel covers these designs");
         }
-        // untuned: the first (tensor-core, else the widest, most specific) one,
-        // and the first staged one
-        auto first_staged = [&] {
+        // Untuned: the first covering one (tensor-core, else the widest, most
+        // specific staged one), and the first staged one.  A tensor-core batch of
+        // at most two tiles (of 1024 coefficients) per SM takes the direct kernel,
+        // which spreads them over more threads, as the plans' own calls take the
+        // window kernel.  Forward, us after an L2 flush / again from L2, staged,
+        // tensor cores and direct: 32 x 32 8.5/6.0, 9.8/3.1, 7.4/2.7; 256 x 1216
+        // 10.8/6.4, 9.3/3.5, 8.4/2.9; 1024 x 304 12.0/8.2, 10.2/3.9, 8.7/3.5;
+        // 1024 x 1216 13.0/8.3, 11.1/4.7, 10.3/6.2; 1024 x 4864 23.8/20.5,
+        // 16.7/9.5, 16.5/10.6; 32 x 2^21 119, 87, 109 (so n = 32 stays here).
+        auto first_of = [&](auto match) {
             size_t c = 0;
-            while (part.layouts[c].cfg.form != BF_STAGED) ++c;   // every family has a staged kernel
+            while (c < part.layouts.size() && !match(part.layouts[c].cfg)) ++c;
             return c;
         };
+        auto first_staged = [&] {                      // every family has a staged kernel
+            return first_of([](const BatchConfig& c) { return c.form == BF_STAGED; });
+        };
         if (flags & GBNTT_BATCH_NO_TUNE) {
-            const size_t c = first_staged();
-            if (c > 1) std::swap(part.layouts[1], part.layouts[c]);
-            part.layouts.resize(c ? 2 : 1);
+            size_t pick = 0;
+            if (part.layouts[0].cfg.form == BF_TC) {
+                long long tiles = 0;
+                for (const auto& pe : part.pending) {
+                    const long long per_tile = TC_TILE >> pe.L;
+                    tiles += ((long long)segs[pe.k].count + per_tile - 1) / per_tile;
+                }
+                if (tiles <= 2 * sms)                  // the 128-thread one holds every length of the tensor cores'
+                    pick = first_of([](const BatchConfig& c) { return c.form == BF_DIRECT && c.cta == 128; });
+            }
+            std::vector<gbntt_batch::Layout> keep = {part.layouts[pick]};
+            if (keep[0].cfg.form != BF_STAGED) keep.push_back(part.layouts[first_staged()]);
+            part.layouts = keep;
         }
         part.staged = (int)first_staged();
         // zero copy: the narrowest covering configuration
@@ -459,9 +482,6 @@ int gbntt_batch_create(gbntt_batch** out, const gbntt_segment* segs, uint32_t ns
         }
       }
     }
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     for (int i = 0; i < b->nparts; ++i) {
         std::vector<gbntt_batch::Layout*> lays;
         for (auto& lay : b->parts[i].layouts) lays.push_back(&lay);

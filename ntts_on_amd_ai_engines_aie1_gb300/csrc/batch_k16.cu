@@ -34,7 +34,8 @@ struct Key {
 // 256-thread CTAs with 64, 32 or 16 coefficients per thread; the narrower
 // ones carry less unrolled code per variant and fit more CTAs per SM (occ:
 // the residency the registers are budgeted for, 0 = the default of the width).
-// The order matters: GBNTT_BATCH_NO_TUNE takes the first covering entry.
+// The order matters: GBNTT_BATCH_NO_TUNE takes the first covering entry (a
+// canonical batch of few tiles a direct one, batch.cu).
 // (768-thread CTAs, one per SM, measured no faster on GB300.)
 constexpr Key kKeys[] = {
     {6, R4, 0}, {5, R4, 0}, {6, R2, 0}, {5, R2, 0}, {6, R8, 0}, {5, R8, 0}, {5, ALL16, 0},
