@@ -75,11 +75,11 @@ int family_of(int kind) {
     }
 }
 
-KernelInfo kernel_for(int fam, int L, bool br, bool lat) {
+KernelInfo kernel_for(int fam, int L, bool br, bool lat, int form) {
     if (fam_canon(fam)) return kinfo_canon(fam, L, lat);
     switch (fam) {
-    case F_R2F16: return kinfo_r2f16(L, lat);
-    case F_R2I16: return kinfo_r2i16(L, lat);
+    case F_R2F16: return kinfo_r2f16(L, lat, form);
+    case F_R2I16: return kinfo_r2i16(L, lat, form);
     case F_R4F16: return kinfo_r4(L, br, lat);
     case F_R8F16: return kinfo_r8(L, lat);
     case F_R2F32: return kinfo_r2f32(L, lat);
@@ -335,9 +335,10 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
         else p->large = large_info(p->fam, hp.L);
         found = canon ? p->clarge.cols != nullptr : p->large.cols != nullptr;
     }
+    const int form = p->fam == F_R2F16 || p->fam == F_R2I16 ? r2_form(hp.q, hp.c) : R2_WIDE;
     if (p->fam >= 0 && p->two_pass_max != UINT64_MAX) {
-        p->ki = kernel_for(p->fam, hp.L, p->br, false);
-        p->kl = kernel_for(p->fam, hp.L, p->br, true);
+        p->ki = kernel_for(p->fam, hp.L, p->br, false, form);
+        p->kl = kernel_for(p->fam, hp.L, p->br, true, form);
         found = found && p->ki.fn;
     }
     if (!found) {
@@ -382,8 +383,7 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
     }
     // radix-4 and wide radix-2 int16 designs: (tw, w') packed into one word
     // (both fit int16)
-    const int lean = p->fam == F_R2F16 || p->fam == F_R2I16 ? r2_form(hp.q, hp.c) : R2_WIDE;
-    const bool packed = lean == R2_WIDE && (p->fam == F_R2F16 || p->fam == F_R2I16 || p->fam == F_R4F16);
+    const bool packed = form == R2_WIDE && (p->fam == F_R2F16 || p->fam == F_R2I16 || p->fam == F_R4F16);
     const bool inverse = (kind == K_R2_I16_INV || kind == K_R2_I32_INV || kind == K_R4_I16_INV);
     std::vector<int32_t> dev_tab;
     std::vector<uint32_t> tc_tab;
@@ -459,7 +459,7 @@ int gbntt_plan_create(gbntt_plan** out, int kind, uint32_t n, int64_t q, int64_t
     a.c = hp.c;
     a.fneg = hp.r4_fneg;
     a.wc = hp.r4_wc;
-    if (p->fam == F_R2F16 || p->fam == F_R2I16) a.lean = lean;
+    if (p->fam == F_R2F16 || p->fam == F_R2I16) a.lean = form;
     a.canonical = (flags & FLAG_CANONICAL) ? 1 : 0;
     a.canon_c = hp.q >= 3 ? (int)((((uint64_t)1 << 32) + hp.q / 2) / hp.q) : 0;
     if (canon) {

@@ -183,6 +183,7 @@ __device__ __forceinline__ unsigned bm16_lo(int a, int t, int q) {
 //               is left out (w is exact then: the table holds tw and w' apart);
 //   R2_LEAN_ODD and an odd c (12289, 7681): br16_odd.
 enum { R2_WIDE = 0, R2_LEAN = 1, R2_LEAN_ODD = 2 };
+constexpr int R2_ANY = -1;   // of a kernel: the launch's own (KArgs::lean)
 __host__ __device__ constexpr int r2_form(long long q, int c) {
     return q >= 16384 ? R2_WIDE : c & 1 ? R2_LEAN_ODD : R2_LEAN;
 }
@@ -1162,23 +1163,29 @@ __device__ __forceinline__ void ntt_tile(const KArgs& a, int lean, long long pol
     if (active) store_poly<I32, L, EL, LOZ>(v, a, poly, g);
 }
 
-template <int FAM, int L, int EL, int P, bool BR>
+template <int FAM, int L, int EL, int P, bool BR, int FORM>
 __device__ __forceinline__ void k_ntt_body(const KArgs& a) {
     extern __shared__ int smem[];
     // Every stage's table loads sit on the transform's dependent path; in a
     // launch of a few polynomials (latency) they would wait stage by stage, so
     // the host asks for the whole table in L1 first, beside the polynomial's load.
     const char* tb = a.tab16 ? reinterpret_cast<const char*>(a.tab16) : reinterpret_cast<const char*>(a.tab);
-    for (int off = (int)threadIdx.x * 128; off < a.tab_bytes; off += (int)blockDim.x * 128)
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(tb + off));
-    ntt_tile<FAM, L, EL, P, BR>(a, a.lean, (long long)blockIdx.x * P, smem);
+    if constexpr (L <= 3) {
+        // a thread does it without a loop, which costs n = 8 a tenth (us over 2^25
+        // coefficients, canonical inverse 30.0 for 32.1, with n^-1 28.8 for 32.4)
+        if ((int)threadIdx.x * 128 < a.tab_bytes) asm volatile("prefetch.global.L1 [%0];" ::"l"(tb + threadIdx.x * 128));
+    } else {
+        for (int off = (int)threadIdx.x * 128; off < a.tab_bytes; off += (int)blockDim.x * 128)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(tb + off));
+    }
+    ntt_tile<FAM, L, EL, P, BR>(a, FORM == R2_ANY ? a.lean : FORM, (long long)blockIdx.x * P, smem);
 }
 
 // MB: resident CTAs per SM the registers are budgeted for (kntt_min_blocks)
-template <int FAM, int L, int EL, int P, bool BR, int MB>
+template <int FAM, int L, int EL, int P, bool BR, int MB, int FORM = R2_ANY>
 __global__ void __launch_bounds__(P << (L - EL), MB) k_ntt(const __grid_constant__ KArgs a) {
     grid_dep_start();
-    k_ntt_body<FAM, L, EL, P, BR>(a);
+    k_ntt_body<FAM, L, EL, P, BR, FORM>(a);
 }
 
 struct KernelInfo {
@@ -1199,23 +1206,31 @@ struct KernelInfo {
 //     1.75);
 //   * 128-thread CTAs where a polynomial needs no more: an exchange then waits
 //     for four warps, not eight (canonical int32 n = 2048 forward 3.49 for
-//     3.05, lanes 2.49 for 2.45, radix-4 n = 1024 1.98 for 1.95);
+//     3.05, lanes 2.49 for 2.45, radix-4 n = 1024 1.98 for 1.95).  Up to n = 8,
+//     where a thread has a polynomial of its own and at most 16 bytes of int16,
+//     CTAs start one a nanosecond and 128 threads of work are less than that:
+//     256 (us over 2^25 coefficients: n = 2 71 for 135, n = 4 int16 38.5 for 70,
+//     int32 47 for 70, canonical int16 n = 8 30-31 for 37);
 //   * 48 registers a thread at 16 coefficients, 64 to 72 at 32: left to the
 //     compiler, the code takes 56 to 104 and half the warps fit (radix-2 int16
-//     n = 4096 forward 1.27 for 1.66, int32 n = 2048 lanes 1.90 for 2.49).
+//     n = 4096 forward 1.27 for 1.66, int32 n = 2048 lanes 1.90 for 2.49);
+//   * 32 registers at 8 coefficients and fewer.  The radix-2 int16 inverse of n =
+//     64 has 8: 2^25 coefficients in 50.8 us (q = 12289) and 59.0 (a modulus
+//     above 2^14), 55.5 and 63.0 with 46 registers, 72 and 73 with 16 coefficients.
 __host__ __device__ constexpr int choose_el(int fam, int L) {
     if (L <= 5) return L;
-    if (fam == F_R2I16) return L >= 9 ? 5 : 4;
+    if (fam == F_R2I16) return L >= 9 ? 5 : L == 6 ? 3 : 4;
     if (fam == F_C16I && L == 12) return 5;
     return L == 13 || L == 15 ? 5 : 4;
 }
 __host__ __device__ constexpr int choose_polys(int fam, int L) {
     const int G = 1 << (L - choose_el(fam, L));
-    const int p = 128 / G;
+    const int p = (L <= 3 ? 256 : 128) / G;
     return p < 1 ? 1 : p;
 }
 __host__ __device__ constexpr int kntt_min_blocks(int fam, int threads, int el) {
     if (el >= 5) return threads <= 128 ? 7 : threads <= 256 ? 4 : threads <= 512 ? 2 : 1;
+    if (el <= 3 && threads <= 256) return 2048 / threads;
     if (threads <= 128) return 10;
     // n = 4096: 40 registers for the radix-4 and canonical code (radix-4 1.69
     // for 1.62, canonical int32 forward 3.91 for 3.82, inverse 4.09 for 4.03)
@@ -1238,13 +1253,13 @@ __host__ __device__ constexpr bool has_lat(int fam, int L) {
     return L >= 9 && L <= 12 && (lat_el(fam, L) != choose_el(fam, L) || choose_polys(fam, L) != 1);
 }
 
-template <int FAM, int L, bool BR, bool LAT = false>
+template <int FAM, int L, bool BR, bool LAT = false, int FORM = R2_ANY>
 KernelInfo make_kernel_info() {
     constexpr int EL = LAT ? lat_el(FAM, L) : choose_el(FAM, L);
     constexpr int P = LAT ? 1 : choose_polys(FAM, L);
     KernelInfo ki;
     constexpr int MB = LAT ? 1 : kntt_min_blocks(FAM, P << (L - EL), EL);
-    ki.fn = reinterpret_cast<const void*>(&k_ntt<FAM, L, EL, P, BR, MB>);
+    ki.fn = reinterpret_cast<const void*>(&k_ntt<FAM, L, EL, P, BR, MB, FORM>);
     ki.threads = P << (L - EL);
     ki.smem = num_windows(FAM, L, EL) > 1 ? P * xwords(L) * 4 : 0;
     ki.polys = P;
@@ -1253,9 +1268,10 @@ KernelInfo make_kernel_info() {
 }
 
 // kernel tables, one per family (kernels_*.cu)
-// lat: the latency form (an empty KernelInfo where the design has none)
-KernelInfo kinfo_r2f16(int L, bool lat);
-KernelInfo kinfo_r2i16(int L, bool lat);
+// lat: the latency form (an empty KernelInfo where the design has none);
+// form: of the plan's radix-2 int16 butterflies
+KernelInfo kinfo_r2f16(int L, bool lat, int form);
+KernelInfo kinfo_r2i16(int L, bool lat, int form);
 KernelInfo kinfo_r2f32(int L, bool lat);
 KernelInfo kinfo_r2g32(int L, bool lat);
 KernelInfo kinfo_r4(int L, bool br, bool lat);
