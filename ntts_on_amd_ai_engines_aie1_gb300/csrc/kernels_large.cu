@@ -30,6 +30,20 @@ __host__ __device__ constexpr int large_cols(int L1) {
     return c < 32 ? 32 : c;
 }
 
+// Rows per CTA: one, and for the inverse, whose first pass this is, as many as
+// make 128 threads, with registers for six such CTAs per SM.  With 64 threads (2^17) and
+// 32 (2^14) short calls took 4 us longer: 2 / 4 / 8 polynomials of 2^17 11.1 /
+// 11.6 / 15.2 us for 16.9 / 17.0 / 19.1, 16 / 64 of 2^14 10.9 / 14.6 for 14.9 /
+// 18.0; 512 of 2^17 369 for 369 (373 with registers for ten).  The forward's rows,
+// its second pass, do not gain (8 of 2^17 17.3 for 15.9).
+__host__ __device__ constexpr int large_rows(int fam, int L2) {
+    const int G = 1 << (L2 - LARGE_EL);
+    return topdown(fam) || G >= 128 ? 1 : 128 / G;
+}
+__host__ __device__ constexpr int large_row_blocks(int fam, int L2, int rows) {
+    return rows > 1 ? 6 : kntt_min_blocks(fam, 1 << (L2 - LARGE_EL), LARGE_EL);
+}
+
 // one CTA: COLS adjacent columns of one polynomial, G threads per column
 template <int FAM, int L1, int COLS>
 __global__ void __launch_bounds__(COLS << (L1 - large_el(L1)), kntt_min_blocks(FAM, COLS << (L1 - large_el(L1)), LARGE_EL))
@@ -59,7 +73,7 @@ __global__ void __launch_bounds__(COLS << (L1 - large_el(L1)), kntt_min_blocks(F
 
 // one CTA: P rows of 2^L2 coefficients, G threads per row
 template <int FAM, int L2, int P>
-__global__ void __launch_bounds__(P << (L2 - LARGE_EL), kntt_min_blocks(FAM, P << (L2 - LARGE_EL), LARGE_EL))
+__global__ void __launch_bounds__(P << (L2 - LARGE_EL), large_row_blocks(FAM, L2, P))
     k_rows(const __grid_constant__ KArgs a, int L1) {
     constexpr int EL = LARGE_EL, G = 1 << (L2 - EL), E = 1 << EL, NS = nsteps(FAM, L2), N = 1 << L2;
     constexpr int LO0 = window_lo(FAM, L2, EL, 0), LOZ = window_lo(FAM, L2, EL, NS - 1);
@@ -93,7 +107,7 @@ LargeInfo make_large() {
     li.cols_threads = C << (L1 - EL1);
     li.cols_smem = num_windows(FAM, L1, EL1) > 1 ? C * (1 << L1) * 4 : 0;
     li.cols_per_cta = C;
-    constexpr int G2 = 1 << (L2 - LARGE_EL), P = 1;
+    constexpr int G2 = 1 << (L2 - LARGE_EL), P = large_rows(FAM, L2);
     li.rows = reinterpret_cast<const void*>(&k_rows<FAM, L2, P>);
     li.rows_threads = P * G2;
     li.rows_smem = P * xwords(L2) * 4;
