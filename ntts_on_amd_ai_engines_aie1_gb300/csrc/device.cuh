@@ -147,6 +147,12 @@ __host__ __device__ __forceinline__ int rsz32(int a, int b) {
     return (int)(((long long)a * b + (long long)(unsigned long long)bias) >> 32);
 }
 
+// the same with the sign read off the product: a 64-bit addition more, no exclusive or
+__host__ __device__ __forceinline__ int rsz32p(int a, int b) {
+    const long long p = (long long)a * b;
+    return (int)((p + 0x7FFFFFFFLL + (long long)((unsigned long long)p >> 63)) >> 32);
+}
+
 // round(a b / 2^31), ties toward zero (bias and sign as in rsz32)
 __host__ __device__ __forceinline__ int rsz31(int a, int b) {
     const unsigned bias = 0x3FFFFFFFu + ((unsigned)(a ^ b) >> 31);
@@ -184,6 +190,15 @@ __device__ __forceinline__ unsigned bm16_lo(int a, int t, int q) {
 //   R2_LEAN_ODD and an odd c (12289, 7681): br16_odd.
 enum { R2_WIDE = 0, R2_LEAN = 1, R2_LEAN_ODD = 2 };
 constexpr int R2_ANY = -1;   // of a kernel: the launch's own (KArgs::lean)
+// Of the int32 lanes and the canonical int16 families: the code of the staged
+// batch kernel, which has 64 and 40 registers a thread and its tiles in shared
+// memory.  Over 2^25 coefficients there, us, with / without: the rounding's sign
+// read off the product, int32 n = 4 78.6 / 82.1, 4096 135.6 / 138.1 and 138.1 /
+// 144.3 (the direct and per-plan kernels: within 3 % either way); 2q formed where
+// it is used, and no vector loads of the table in the canonical int16 forward
+// (124 bytes of spills without both, 4 with), forward n = 16 58.7 / 60.0, 32 69.9 / 72.9,
+// inverse 32 75.2 / 77.1, 2048 79.3 / 82.8.
+constexpr int FORM_STAGED = 3;
 __host__ __device__ constexpr int r2_form(long long q, int c) {
     return q >= 16384 ? R2_WIDE : c & 1 ? R2_LEAN_ODD : R2_LEAN;
 }
@@ -195,12 +210,15 @@ __device__ __forceinline__ void r2_butterfly16(int& x, int& y, int2 t, int c, in
     y = u - w;
 }
 
-// int32 variants, computed modulo 2^32 like the int32 lanes
+// int32 variants, computed modulo 2^32 like the int32 lanes (FORM_STAGED: with rsz32p)
+template <int FORM = R2_WIDE>
 __host__ __device__ __forceinline__ int br32(int a, int c, int q) {
-    return (int)((unsigned)a - (unsigned)rsz32(a, c) * (unsigned)q);
+    return (int)((unsigned)a - (unsigned)(FORM == FORM_STAGED ? rsz32p(a, c) : rsz32(a, c)) * (unsigned)q);
 }
+template <int FORM = R2_WIDE>
 __host__ __device__ __forceinline__ int bm32(int a, int tw, int wq, int q) {
-    return (int)((unsigned)a * (unsigned)tw - (unsigned)rsz32(a, wq) * (unsigned)q);
+    return (int)((unsigned)a * (unsigned)tw -
+                 (unsigned)(FORM == FORM_STAGED ? rsz32p(a, wq) : rsz32(a, wq)) * (unsigned)q);
 }
 __device__ __forceinline__ int add32(int a, int b) { return (int)((unsigned)a + (unsigned)b); }
 __device__ __forceinline__ int sub32(int a, int b) { return (int)((unsigned)a - (unsigned)b); }
@@ -645,7 +663,7 @@ __device__ __forceinline__ void exchange_cols(int (&v)[1 << EL], int* sp, int g,
 // 2^B .. 2^(B+1) - 1, when the window is the lowest bits
 template <int FAM, int FORM>
 __host__ __device__ constexpr int step_vec_pairs(int LO, int EL, int B, bool HIB) {
-    if (LO != 0) return 0;
+    if (LO != 0 || (FORM == FORM_STAGED && FAM == F_C16F)) return 0;
     if (fam_canon(FAM) && !HIB) return B >= 1 && B < EL ? 1 << B : 0;
     const bool blocks = fam_canon(FAM) || FAM == F_R2F32 || FAM == F_R2G32 || (FAM == F_R2F16 && FORM != R2_WIDE);
     const int n = (1 << EL) >> (B + 1);
@@ -735,7 +753,7 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
             const int k1 = k0 | (1 << KB);
             // 2q comes as a value of its own: from q, every x + 2q - y
             // becomes a shift-and-add and a subtraction
-            const unsigned uq = (unsigned)q, q2 = (unsigned)a.c;
+            const unsigned uq = (unsigned)q, q2 = FORM == FORM_STAGED && !fam_i32(FAM) ? uq << 1 : (unsigned)a.c;
             if constexpr (topdown(FAM)) {
                 // Forward: Gentleman-Sande, natural order in, bit-reversed out.
                 // Layer S pairs the positions differing in bit B = L-1-S:
@@ -809,7 +827,7 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
                 v[k1] = wrap16((int)(u - w));
             } else {
                 const int2 t = NV > 0 ? tv[k0 >> (B + 1)] : __ldg(&a.tab[blk]);
-                const int u = br32(v[k0], a.c, q), w = bm32(v[k1], t.x, t.y, q);
+                const int u = br32<FORM>(v[k0], a.c, q), w = bm32<FORM>(v[k1], t.x, t.y, q);
                 v[k0] = add32(u, w);
                 v[k1] = sub32(u, w);
             }
@@ -819,8 +837,8 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
             const int blk = ((HIB ? (hi << L) : 0) | posmap<LO, EL>(g, k0)) >> (B + 1);
             const int2 t = NV > 0 ? tv[k0 >> (B + 1)] : __ldg(&a.tab[blk]);
             const int s = add32(v[k0], v[k1]), d = sub32(v[k0], v[k1]);
-            v[k0] = br32(s, a.c, q);
-            v[k1] = bm32(d, t.x, t.y, q);
+            v[k0] = br32<FORM>(s, a.c, q);
+            v[k1] = bm32<FORM>(d, t.x, t.y, q);
         } else if constexpr (FAM == F_R2I16) {
             // inverse CT layer S on bit-reversed input (ntt_r2_kernels.cc:484-540)
             const int k1 = k0 | (1 << KB);
@@ -930,8 +948,9 @@ __device__ __forceinline__ void do_step(int (&v)[1 << EL], int* sp, int g, const
     }
 }
 
-// lean: the form of radix-2 int16 butterflies (the same for the whole CTA)
-template <int FAM, int L, int EL, int... S>
+// lean: the form of radix-2 int16 butterflies (the same for the whole CTA);
+// FORM: of the other families (FORM_STAGED, or R2_WIDE)
+template <int FAM, int L, int EL, int FORM = R2_WIDE, int... S>
 __device__ __forceinline__ void run_steps(int (&v)[1 << EL], int* sp, int g, const KC& a, int lean, bool fresh,
                                           std::integer_sequence<int, S...>) {
     if constexpr (FAM == F_R2F16 || FAM == F_R2I16) {
@@ -944,7 +963,8 @@ __device__ __forceinline__ void run_steps(int (&v)[1 << EL], int* sp, int g, con
             return;
         }
     }
-    (do_step<FAM, L, EL, S>(v, sp, g, a, 0, 0, fresh), ...);
+    constexpr int F = FAM == F_R2F16 || FAM == F_R2I16 ? R2_WIDE : FORM;
+    (do_step<FAM, L, EL, S, 0, false, F>(v, sp, g, a, 0, 0, fresh), ...);
 }
 
 template <int FAM, int L, int EL, int XC, bool HIB, int... S>

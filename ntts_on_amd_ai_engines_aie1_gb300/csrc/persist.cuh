@@ -231,7 +231,7 @@ __device__ __forceinline__ void tile_transform(void* stage, int* xbuf, const KC&
             fresh = false;
         }
     }
-    run_steps<FAM, L, EL>(v, sp, g, a, ka.lean, fresh, std::make_integer_sequence<int, NS>{});
+    run_steps<FAM, L, EL, FORM_STAGED>(v, sp, g, a, ka.lean, fresh, std::make_integer_sequence<int, NS>{});
     epilogue<FAM, false>(v, ka);
     if (!active) return;
     if constexpr (fam_natural_out(FAM, false)) {

@@ -37,3 +37,7 @@ def test_lane_rounding(tmp_path):
 
 def test_two_pass_tables(tmp_path):
     _run_host_check(tmp_path, "two_pass_tables")
+
+
+def test_staged_rounding(tmp_path):
+    _run_host_check(tmp_path, "staged_rounding")
