@@ -93,7 +93,9 @@ typedef enum gbntt_status {
  * (Shoup multiplication by precomputed quotients, lazily reduced 32-bit lanes,
  * one reduction at the end; twiddle tables built on the device), for every
  * transform design except the radix-8 single stage and the radix-8 chain with
- * the reference's float multipliers, and int32 moduli below 2^30.
+ * the reference's float multipliers, and int32 moduli below 2^30.  Inputs may
+ * be any int16 or int32 value; int32 ones that are residues already (below 2 q)
+ * skip the reduction on load: calls with others take 2 to 9 % longer.
  * GBNTT_FLAG_CANONICAL | GBNTT_FLAG_LANE_EXACT: the reference's own lane
  * arithmetic (the default partial kernels, wraps included) reduced to [0, q),
  * i.e. exactly the reference's residues also where its lanes wrap (full-range
@@ -213,7 +215,9 @@ typedef struct gbntt_batch gbntt_batch;
  * inputs and outputs fit in L2 is timed from HBM: creation then briefly
  * allocates twice the L2 size of scratch to evict it between the timed
  * launches (without room for it, the launches are timed back to back).
- * Creation then writes the segments' outputs. */
+ * Creation then writes the segments' outputs.  Untuned batches take a staged
+ * configuration, canonical int16 ones of n = 2^5 .. 2^10 the tensor-core kernel
+ * beyond two tiles of 1024 coefficients per SM and the direct one up to them. */
 #define GBNTT_BATCH_NO_TUNE 0x1u
 int gbntt_batch_create(gbntt_batch** batch, const gbntt_segment* segs, uint32_t nsegs, uint32_t flags);
 int gbntt_batch_execute(gbntt_batch* batch, void* stream);
@@ -224,7 +228,7 @@ int gbntt_batch_graph_launch(gbntt_batch* batch, void* stream);
  * address space (cudaHostAlloc / cudaHostRegister memory, 16-byte aligned),
  * the zero-copy form of the persistent kernel reads and writes them directly
  * over the host-device link, so inbound and outbound traffic overlap (one
- * launch per storage type; h_in[i] == h_out[i] allowed; a call on the same
+ * launch per storage type and arithmetic; h_in[i] == h_out[i] allowed; a call on the same
  * buffers as the previous successful one reuses the descriptors already on
  * the device); the other segments are copied through their device buffers.
  * Otherwise copies h_in[i] into
@@ -302,8 +306,8 @@ int gbntt_noalloc_status(void);
  * capped at half of the HBM free at creation), groups the waiting ones by
  * plan into a micro-batch per free stream slot, and overlaps the copies and
  * kernels of up to `slots` micro-batches.  A micro-batch is one in-place
- * launch of the persistent kernel per storage type covering all its plan
- * groups (int32 n >= 2^16 and the radix-4 inverse, bit-reversal and full
+ * launch of the persistent kernel per storage type and arithmetic covering all its plan
+ * groups (int32 n >= 2^14 and the radix-4 inverse, bit-reversal and full
  * Barrett designs: their plans' own launches).  Page-locked host buffers
  * mapped into the device's address space are read and written by a gather and
  * a scatter kernel (no per-request copy call); other host memory goes through

@@ -279,7 +279,8 @@ class Plan:
 
 
 class Batch:
-    """Many polynomials of several designs in one persistent launch.
+    """Many polynomials of several designs in one launch per storage type and
+    arithmetic, on the fastest of three kernels (timed at creation).
 
     segments: list of (plan, input tensor, output tensor); the tensors' first
     dimension (or numel / n) gives the polynomial count.  The batch keeps

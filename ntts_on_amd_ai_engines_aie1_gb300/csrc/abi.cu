@@ -39,7 +39,7 @@ struct gbntt_plan {
     size_t tab_bytes = 0;
     size_t tile_tab_bytes = 0;   // of these, the table of the one-CTA kernels (first in d_tab)
     size_t tc_bytes = 0;   // tensor-core table behind it in the same allocation
-    const void* tc_fn = nullptr;   // tensor-core kernel (canonical int16, n = 2^5 .. 2^10)
+    const void* tc_fn = nullptr;   // tensor-core kernel (canonical int16, n = 2^6 .. 2^10)
     int device = 0;
     std::mutex stage_mu;   // serialises gbntt_execute_host on this plan
     void* d_stage = nullptr;

@@ -1,5 +1,6 @@
-// batch.cu -- persistent batched launches (gbntt_batch_* in include/gb300_ntt.h):
-// segment descriptors, tile order, configuration autotuning, graph replay.
+// batch.cu -- batched launches (gbntt_batch_* in include/gb300_ntt.h) on the staged,
+// the direct and the tensor-core batch kernels: segment descriptors, tile order,
+// configuration autotuning, graph replay, and the zero-copy calls.
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -20,7 +21,7 @@ using namespace gbntt;
 using namespace gbntt;
 
 struct gbntt_batch {
-    struct Layout {                     // one configuration of one persistent launch
+    struct Layout {                     // one configuration of one part's launch
         BatchConfig cfg{};
         std::vector<SegDev> segs;
         SegDev* d_segs = nullptr;
@@ -44,7 +45,7 @@ struct gbntt_batch {
         std::vector<int> user_index;    // caller's segment of each SegDev
         Layout zlay;                    // zero-copy launch (k_batch_zc), when a configuration has one
     };
-    Part parts[BATCH_PARTS];            // one persistent launch per storage type and arithmetic
+    Part parts[BATCH_PARTS];            // one launch per storage type and arithmetic
     int nparts = 0;
     std::vector<int> part_of;           // segment -> part (or -1: separate per-plan launch)
     std::vector<int> index_in_part;

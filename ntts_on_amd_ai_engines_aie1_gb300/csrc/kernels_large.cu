@@ -1,4 +1,4 @@
-// kernels_large.cu -- int32 transforms of 2^16 .. 2^22 coefficients in two passes.
+// kernels_large.cu -- int32 lane transforms of 2^14 .. 2^22 coefficients in two passes.
 //
 // The reference's layers are in-place butterflies on position bits (see
 // device.cuh).  For n = 2^(L1 + L2), the forward layers on the L1 high bits
@@ -21,8 +21,8 @@ constexpr int LARGE_EL = 4;
 __host__ __device__ constexpr int large_el(int L) { return L < LARGE_EL ? L : LARGE_EL; }
 // At least 32 columns (128-byte accesses) and 256 threads per CTA.  Rows are
 // 2^12 coefficients (2^13 for n = 2^22), as long as the row pass runs well;
-// columns are the rest, so that their pass has two windows at most.  2^14, 2^17
-// and 2^18 measured faster with shorter rows (over 2^26 coefficients, forward /
+// columns are the rest, so that their pass has two windows at most and at least
+// four bits.  2^14, 2^17 and 2^18 measured faster with shorter rows (over 2^26 coefficients, forward /
 // inverse: 2^17 5+12 391/406 us, 7+10 390/386; 2^18 6+12 410/421, 7+11 408/409;
 // 64 polynomials of 2^14, 4+10 16/13 us, 5+9 14/13).
 __host__ __device__ constexpr int large_cols(int L1) {
